@@ -177,7 +177,8 @@ VL_API int vl_run_state_init(vl_ctx *ctx, vl_run_state *state, const double *E0,
  * bookkeeping (ts:91-103), entirely on the device: each step runs only while
  * state->time < final_time and steps < max_steps (checked on the device, so extra steps
  * in a batch are no-ops).  f is advanced in place.  stage_a / stage_b are state-sized
- * buffers whose velocity-ghost elements must equal f's (vl_sync_ghosts does that).
+ * buffers whose velocity-ghost elements must equal f's (vl_sync_ghosts
+ * or vl_sync_stage_ghosts does that).
  * E / phi receive the last field solved (of RK stage s1, as in the reference).             */
 VL_API int vl_ssp_rk3_steps(vl_ctx *ctx, void *f, void *stage_a, void *stage_b, double *E,
                      double *phi, vl_run_state *state, void *workspace, int nsteps,
@@ -208,6 +209,16 @@ VL_API int vl_set_background_pairs(vl_ctx *ctx, const float *pairs);
  * reference's periodic x-ghost swap on f (Distribution.swap_ghost_cells_of_array,
  * main/grid.py:187-189).  Call once before a run and after f is replaced.                  */
 VL_API int vl_sync_ghosts(vl_ctx *ctx, void *f, void *stage, void *stream);
+
+/* What vl_ssp_rk3_steps needs of its buffers before a run, without passes over the interior: the
+ * periodic x-ghost swap on f, and f's velocity-ghost elements (of every interior x element)
+ * copied into both stage buffers.  The rest of the stage buffers is left as it is.           */
+VL_API int vl_sync_stage_ghosts(vl_ctx *ctx, void *f, void *stage_a, void *stage_b, void *stream);
+
+/* vl_rhs (weights NULL) or vl_rhs_weighted into an uninitialised array: the interior as they write
+ * it, every ghost element (x, u and v) zero.                                                 */
+VL_API int vl_rhs_whole(vl_ctx *ctx, const void *f, const double *E, void *out, int xhalo,
+                        const double *weights, void *stream);
 
 /* ---- the DG Poisson solve and the linear SSP-RK stepper's interior update ------------------- */
 

@@ -24,6 +24,7 @@ EXPORTED = (
     "vl_ctx_create", "vl_ctx_destroy", "vl_last_error", "vl_abi_version", "vl_state_elems",
     "vl_workspace_bytes", "vl_rhs", "vl_rhs_weighted", "vl_moment", "vl_poisson", "vl_field_energy", "vl_adapt_dt",
     "vl_rk_stage", "vl_run_state_init", "vl_ssp_rk3_steps", "vl_sync_ghosts",
+    "vl_sync_stage_ghosts", "vl_rhs_whole",
     "vl_ssp_rk3_steps_noalloc", "vl_initial_state", "vl_smooth_edges", "vl_interpolate",
     "vl_set_background", "vl_set_background_pairs", "vl_ens_create", "vl_ens_destroy", "vl_ens_workspace_bytes", "vl_ens_bind",
     "vl_ens_schedule", "vl_ens_schedule_by_order", "vl_ens_commit", "vl_ens_steps", "vl_mlp_dims", "vl_mlp_forward",
@@ -102,6 +103,8 @@ def _declare(lib):
                                       ctypes.c_int32, vp, vp]
     lib.vl_ssp_rk3_steps.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i, vp]
     lib.vl_sync_ghosts.argtypes = [vp, vp, vp, vp]
+    lib.vl_sync_stage_ghosts.argtypes = [vp, vp, vp, vp, vp]
+    lib.vl_rhs_whole.argtypes = [vp, vp, vp, vp, i, vp, vp]
     lib.vl_ssp_rk3_steps_noalloc.argtypes = [vp, vp, vp, vp, vp, vp, vp, i, vp]
     i32 = ctypes.c_int32
     lib.vl_set_background.argtypes = [vp, vp, vp]

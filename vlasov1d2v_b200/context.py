@@ -140,6 +140,16 @@ class NativeContext:
         _lib.call("vl_rhs_weighted", self.handle, _ptr(f), _ptr(E), _ptr(out), int(xhalo),
                   ctypes.cast(w, ctypes.POINTER(ctypes.c_double)), ctypes.c_void_p(stream_handle()))
 
+    def rhs_whole(self, f, E, out, weights=None, xhalo=_lib.VL_XHALO_GHOST):
+        """The right-hand side (direction weights: ``rhs_weighted``) with zero ghost elements, into
+        an uninitialised ``out``."""
+        self._check_state(f, "f")
+        self._check_state(out, "out")
+        self._check_field(E, (self.nx + 2, self.n), "E")
+        w = None if weights is None else (ctypes.c_double * 3)(*[float(x) for x in weights])
+        _lib.call("vl_rhs_whole", self.handle, _ptr(f), _ptr(E), _ptr(out), int(xhalo), w,
+                  ctypes.c_void_p(stream_handle()))
+
     def moment(self, f, rho):
         self._check_state(f, "f")
         self._check_field(rho, (self.nx, self.n), "rho")
@@ -185,6 +195,13 @@ class NativeContext:
         if stage is not None:
             self._check_state(stage, "stage")
         _lib.call("vl_sync_ghosts", self.handle, _ptr(f), _ptr(stage), ctypes.c_void_p(stream_handle()))
+
+    def sync_stage_ghosts(self, f, sa, sb):
+        self._check_state(f, "f")
+        self._check_state(sa, "stage_a")
+        self._check_state(sb, "stage_b")
+        _lib.call("vl_sync_stage_ghosts", self.handle, _ptr(f), _ptr(sa), _ptr(sb),
+                  ctypes.c_void_p(stream_handle()))
 
     def run_state_init(self, state, E0, final_time, max_steps, energy_hist, time_hist, dt_hist,
                        energy0=None):

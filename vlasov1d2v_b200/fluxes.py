@@ -2,7 +2,8 @@
 
 Mirrors ``DGFlux`` of crewsdw/Vlasov1D2V (``main/fluxes.py:13-207``).  The whole operator --
 flux products, the three ``up`` contractions, the upwind face fluxes in x, u and v with the
-lift, and the Jacobian-weighted sum -- is one native kernel launch (``vl_rhs``).
+lift, and the Jacobian-weighted sum -- is one native kernel launch, the zero ghost elements of the
+result another (``vl_rhs_whole``).
 """
 from __future__ import annotations
 
@@ -32,11 +33,8 @@ class DGFlux:
         f = _device.as_tensor(function).contiguous()
         ctx = self._ctx(f, elliptic, grids)
         E = _device.as_tensor(elliptic.electric_field, dtype=torch.float64).contiguous()
-        out = torch.zeros_like(f)
-        if weights is None:
-            ctx.rhs(f, E, out, xhalo=_lib.VL_XHALO_GHOST)
-        else:
-            ctx.rhs_weighted(f, E, out, weights, xhalo=_lib.VL_XHALO_GHOST)
+        out = torch.empty_like(f)
+        ctx.rhs_whole(f, E, out, weights, xhalo=_lib.VL_XHALO_GHOST)
         return _device.wrap(out)
 
     def semi_discrete_rhs(self, function, elliptic, basis, grids):

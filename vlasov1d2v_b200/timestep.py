@@ -86,8 +86,7 @@ class _Run:
         return _lib.VlRunState.from_buffer_copy(raw)
 
     def sync_ghosts(self):
-        self.ctx.sync_ghosts(self.f, self.sa)
-        self.ctx.sync_ghosts(self.f, self.sb)
+        self.ctx.sync_stage_ghosts(self.f, self.sa, self.sb)
         self.synced_ptr = self.f.data_ptr()
 
     def launch(self, nsteps, use_graph):
