@@ -24,6 +24,7 @@
 #include "vlasov_stage_frag.cuh"
 #include "vlasov_stage_f32.cuh"
 #include "vlasov_field.cuh"
+#include "vlasov_field_conv.cuh"
 #include "vlasov_stage_gen.cuh"
 #include "vlasov_gen_kinds.h"
 
@@ -766,6 +767,8 @@ vl::FieldArgs field_args(const vl_ctx *c) {
     a.phase = c->d_phase;
     a.qnode = c->d_qnode;
     a.k = c->d_k;
+    a.KE = c->d_ke;
+    a.KP = c->d_kp;
     a.xw = c->d_xw;
     a.nx = c->cfg.nx;
     a.n = c->cfg.n;
@@ -783,8 +786,55 @@ vl::FieldArgs field_args(const vl_ctx *c) {
     return a;
 }
 
+// the solve as a convolution (vlasov_field_conv.cuh)
+int field_conv(const vl::FieldArgs &a, cudaStream_t s) {
+    const size_t smem = vl::field_conv_smem(a.nx, a.n, a.phi != nullptr);
+    if (!(a.mode & vl::FIELD_RECORD)) {
+        vl::field_conv_kernel<<<a.nx, vl::FV_THREADS, smem, s>>>(a);
+        return check_launch("field_conv_kernel");
+    }
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(vl::FC);
+    cfg.blockDim = dim3(vl::FV_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = vl::FC;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return check_launch(cudaLaunchKernelEx(&cfg, vl::field_conv_record_kernel, a), "field_conv_record_kernel");
+}
+
+// whether conj(ph[e, m]) ph[e', m] depends on (e - e') mod nx only, to the rounding of the phases
+// (k_m x up to 2.5 pi nx: below 5e-13)
+bool uniform_phases(const vl_config *cfg) {
+    const int nx = cfg->nx, M = cfg->n_modes;
+    const double *ph = cfg->dft_phase;
+    const double tol = 2e-12;
+    for (int m = 0; m < M; ++m) {
+        double r0 = 0.0, r1 = 0.0;
+        for (int e = 0; e < nx; ++e) {
+            const double *a = ph + 2 * ((size_t)e * M + m), *b = ph + 2 * ((size_t)((e + 1) % nx) * M + m);
+            if (!(std::fabs(a[0] * a[0] + a[1] * a[1] - 1.0) < tol)) return false;
+            const double c = a[0] * b[0] + a[1] * b[1], s = a[0] * b[1] - a[1] * b[0];
+            if (e == 0) {
+                r0 = c;
+                r1 = s;
+            } else if (!(std::fabs(c - r0) < tol && std::fabs(s - r1) < tol)) {
+                return false;
+            }
+        }
+    }
+    return true;
+}
+
 // the whole spectral solve in one thread-block cluster of vl::FC CTAs (vlasov_field.cuh)
 int field(const vl_ctx *c, const vl::FieldArgs &a0, cudaStream_t s) {
+    if (a0.KE != nullptr) return field_conv(a0, s);
     // the table prefetch where it fits the dynamic shared memory budget
     vl::FieldArgs a = a0;
     const size_t base = vl::field_solve_smem_for(a.n, a.M, a.phi != nullptr);
@@ -970,6 +1020,27 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
             (int)std::max(vl::field_solve_smem(vl::NMAX, vl::FIELD_MAX_MODES), vl::FIELD_DYN_SMEM_MAX));
         if (ee != cudaSuccess) return cleanup(cuda_fail(ee, "cudaFuncSetAttribute(field_solve_kernel)"));
     }
+    // the field solve in its convolution form on a uniform periodic x grid (VLASOV1D2V_FIELD=dft keeps
+    // the transform form, for comparisons)
+    const char *field_env = getenv("VLASOV1D2V_FIELD");
+    if (!(field_env && std::string(field_env) == "dft") && uniform_phases(cfg)) {
+        const size_t kb = sizeof(double) * (size_t)vl::field_conv_elems(cfg->nx, n);
+        cudaError_t ee = cudaMalloc((void **)&c->d_ke, kb);
+        if (ee == cudaSuccess) ee = cudaMalloc((void **)&c->d_kp, kb);
+        if (ee == cudaSuccess) {
+            vl::field_conv_table_kernel<<<(vl::field_conv_elems(cfg->nx, n) + 31) / 32, 256>>>(
+                c->d_ke, c->d_kp, c->d_ell, c->d_phase, c->d_qnode, c->d_k, cfg->nx, n, cfg->n_modes, cfg->dx,
+                cfg->length_x);
+            ee = cudaGetLastError();
+        }
+        if (ee == cudaSuccess) ee = cudaStreamSynchronize(nullptr);
+        const int smem = (int)vl::field_conv_smem(64, vl::NMAX, true);
+        if (ee == cudaSuccess)
+            ee = cudaFuncSetAttribute(vl::field_conv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (ee == cudaSuccess)
+            ee = cudaFuncSetAttribute(vl::field_conv_record_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (ee != cudaSuccess) return cleanup(cuda_fail(ee, "field tables"));
+    }
     {
         std::vector<double> tabs((size_t)2 * n * n + 2 * n);
         std::memcpy(tabs.data(), c->up, sizeof(double) * n * n);
@@ -1077,6 +1148,8 @@ int vl_ctx_destroy(vl_ctx *c) {
     cudaFree(c->d_phase);
     cudaFree(c->d_qnode);
     cudaFree(c->d_tables);
+    cudaFree(c->d_ke);
+    cudaFree(c->d_kp);
     cudaFree(c->d_moment);
     cudaFree(c->d_err);
     delete c;

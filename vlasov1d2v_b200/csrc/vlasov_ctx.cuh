@@ -35,6 +35,8 @@ struct vl_ctx {
     double2 *d_ell = nullptr;     // [n][M]  DFT factors (vl_config dft_ell / dft_phase / dft_qnode)
     double2 *d_phase = nullptr;   // [nx][M]
     double2 *d_qnode = nullptr;   // [n][M]
+    double *d_ke = nullptr;       // convolution form of the field solve (null: the transform form)
+    double *d_kp = nullptr;
     double *d_tables = nullptr;   // up [n n], xi [n 2], qw [n n]
     double *d_moment = nullptr;   // moment partials of vl_moment [nx][moment_grid_g][n]
     int *d_err = nullptr;         // device error word of operators run without a loop state

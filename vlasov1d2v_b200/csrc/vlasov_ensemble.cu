@@ -29,6 +29,7 @@
 
 #include "vlasov_ctx.cuh"
 #include "vlasov_field.cuh"
+#include "vlasov_field_conv.cuh"
 #include "vlasov_stage.cuh"
 
 namespace vl {
@@ -203,6 +204,14 @@ __global__ void __launch_bounds__(FS_THREADS) ens_field_kernel(const FieldArgs *
     field_cluster_body(fa[blockIdx.x / FC]);
 }
 
+// the same in the convolution form: FC CTAs per member, a cluster in the step's last solve only
+__global__ void __launch_bounds__(FV_THREADS) ens_field_conv_kernel(const FieldArgs *__restrict__ fa) {
+    field_conv_body<false>(fa[blockIdx.x / FC], blockIdx.x % FC, FC);
+}
+__global__ void __launch_bounds__(FV_THREADS) ens_field_conv_record_kernel(const FieldArgs *__restrict__ fa) {
+    field_conv_body<true>(fa[blockIdx.x / FC], blockIdx.x % FC, FC);
+}
+
 }  // namespace vl
 
 struct vl_ens {
@@ -237,6 +246,7 @@ struct vl_ens {
     int *d_cta_items = nullptr;
     vl::EnsItem *d_items = nullptr;
     size_t field_smem = 0;   // dynamic shared memory of the field kernel: the largest member's
+    bool conv = false;       // every member's field solve in its convolution form
     bool dirty = true;
 };
 
@@ -385,10 +395,17 @@ int stage(vl_ens *E, int st, cudaStream_t s) {
 
 int field(vl_ens *E, int kind, cudaStream_t s) {
     const int count = (int)E->ctx.size();
+    const vl::FieldArgs *args = E->d_field[kind];
+    if (E->conv && kind != 2) {
+        vl::ens_field_conv_kernel<<<vl::FC * count, vl::FV_THREADS, E->field_smem, s>>>(args);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return efail(VL_ERR_CUDA, std::string("ens_field_conv_kernel: ") + cudaGetErrorString(e));
+        return VL_OK;
+    }
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(vl::FC * count);
-    cfg.blockDim = dim3(vl::FS_THREADS);
+    cfg.blockDim = dim3(E->conv ? vl::FV_THREADS : vl::FS_THREADS);
     cfg.dynamicSmemBytes = E->field_smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -398,7 +415,10 @@ int field(vl_ens *E, int kind, cudaStream_t s) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, vl::ens_field_kernel, static_cast<const vl::FieldArgs *>(E->d_field[kind]));
+    if (E->conv)
+        cudaLaunchKernelEx(&cfg, vl::ens_field_conv_record_kernel, args);
+    else
+        cudaLaunchKernelEx(&cfg, vl::ens_field_kernel, args);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return efail(VL_ERR_CUDA, std::string("ens_field_kernel: ") + cudaGetErrorString(e));
     return VL_OK;
@@ -464,6 +484,8 @@ int commit(vl_ens *E) {
     // order n go to list n (by-order schedule) or all to list 0
     std::vector<CostItem> items[vl::NMAX + 1];
     E->field_smem = 0;
+    E->conv = true;
+    for (const vl_ctx *c : E->ctx) E->conv = E->conv && c->d_ke != nullptr;
     for (int i = 0; i < count; ++i) {
         const vl_ctx *c = E->ctx[i];
         const int G = E->G[i];
@@ -481,7 +503,8 @@ int commit(vl_ens *E) {
         // a member launched through its own context: the solve after the Euler stage reads the
         // partials of that context's Euler-stage grid
         if (E->by_order && E->native[i]) E->field[1][i].G = c->stage_grid_g1;
-        E->field_smem = std::max(E->field_smem, vl::field_solve_smem(c->cfg.n, c->cfg.n_modes));
+        E->field_smem = std::max(E->field_smem, E->conv ? vl::field_conv_smem(c->cfg.nx, c->cfg.n, true)
+                                                        : vl::field_solve_smem(c->cfg.n, c->cfg.n_modes));
     }
     std::vector<int> offs;
     std::vector<vl::EnsItem> flat;
@@ -574,6 +597,9 @@ VL_API int vl_ens_create(vl_ctx *const *ctxs, int32_t count, vl_ens **out) {
     }
     cudaFuncSetAttribute(vl::ens_field_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)vl::field_solve_smem(vl::NMAX, vl::FIELD_MAX_MODES));
+    for (auto *k : {vl::ens_field_conv_kernel, vl::ens_field_conv_record_kernel})
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)vl::field_conv_smem(64, vl::NMAX, true));
     *out = E;
     return VL_OK;
 }
@@ -643,6 +669,8 @@ VL_API int vl_ens_bind(vl_ens *E, int32_t i, void *f, void *sa, void *sb, double
         fa.phase = c->d_phase;
         fa.qnode = c->d_qnode;
         fa.k = c->d_k;
+        fa.KE = c->d_ke;
+        fa.KP = c->d_kp;
         fa.xw = c->d_xw;
         fa.nx = c->cfg.nx;
         fa.n = c->cfg.n;

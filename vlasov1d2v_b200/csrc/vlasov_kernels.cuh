@@ -237,6 +237,8 @@ struct FieldArgs {
     // 1: each CTA first copies the phase-table entries it reads in its loops into shared memory
     // (field_prefetch_bytes more dynamic shared memory; the arithmetic is unchanged)
     int prefetch;
+    // convolution form (vlasov_field_conv.cuh): [nx][field_conv_stride(n)] tables, or null
+    const double *KE, *KP;
 };
 
 constexpr int FIELD_THREADS = 1024;            // threads of the single-CTA scalar kernel
