@@ -664,27 +664,12 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
                 }
                 const bool xpos = uxT >= (T)0;
                 const bool vpos = svT >= (T)0;
-                // x: sum_m up[i][m] F[m][j][k] + lifts
+                // the three contractions' sums advance together: six independent chains.  One contraction
+                // after another, two chains at a time, the FP64 FMA latency bounded the row (n = 9 at
+                // 64^3: 1.84 / 2.02 ms per Euler / combination stage, 1.74 / 1.86 together; FP32 +1%)
+                //   x: sum_m up[i][m] F[m][j][k]    v: sum_m F[i][j][m] up[k][m] (the element's k-line)
+                //   u: sum_m up[j][m] F[i][m][k]    (compile-time j: table constants)
                 const T *pc = rowp(sIn, 0, j) + 2 * p;
-                T dx0 = (T)0, dx1 = (T)0;
-                V2 cm0, cmL;
-#pragma unroll
-                for (int m = 0; m < N; ++m) {
-                    const V2 cv = ld2(pc + m * PIN);
-                    if (m == 0) cm0 = cv;
-                    if (m == N - 1) cmL = cv;
-                    dx0 = fma(upi[m], cv.x, dx0);
-                    dx1 = fma(upi[m], cv.y, dx1);
-                }
-                const V2 xf0 = ld2(facep(sXF, 0, j) + 2 * p);
-                const V2 xf1 = ld2(facep(sXF, 1, j) + 2 * p);
-                const V2 xl = xpos ? xf0 : cm0;
-                const V2 xr = xpos ? cmL : xf1;
-                dx0 = fma(xig0, xl.x, dx0);
-                dx0 = fma(-xig1, xr.x, dx0);
-                dx1 = fma(xig0, xl.y, dx1);
-                dx1 = fma(-xig1, xr.y, dx1);
-                // v: sum_m F[i][j][m] up[k][m] + lifts (the element's k-line)
                 const T *pa = rowp(sIn, i, j);   // k-line of element b
                 T line[2 * P];
 #pragma unroll
@@ -693,28 +678,38 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
                     line[2 * m2] = l2.x;
                     line[2 * m2 + 1] = l2.y;
                 }
-                T dv0 = (T)0, dv1 = (T)0;
+                T dx0 = (T)0, dx1 = (T)0, dv0 = (T)0, dv1 = (T)0, du0 = (T)0, du1 = (T)0;
+                V2 cm0, cmL;
 #pragma unroll
                 for (int m = 0; m < N; ++m) {
+                    const V2 cv = ld2(pc + m * PIN);
+                    if (m == 0) cm0 = cv;
+                    if (m == N - 1) cmL = cv;
+                    dx0 = fma(upi[m], cv.x, dx0);
+                    dx1 = fma(upi[m], cv.y, dx1);
                     dv0 = fma(upk0[m], line[m], dv0);
                     dv1 = fma(upk1[m], line[m], dv1);
-                }
-                const T tl = vpos ? pa[CONTIG ? -1 : LH - H] : line[0];
-                const T tr = vpos ? line[N - 1] : pa[CONTIG ? N : SL];
-                dv0 = fma(xik00, tl, dv0);
-                dv0 = fma(-xik01, tr, dv0);
-                dv1 = fma(xik10, tl, dv1);
-                dv1 = fma(-xik11, tr, dv1);
-                // u: sum_m up[j][m] F[i][m][k] + lifts (compile-time j: table constants)
-                T du0 = (T)0, du1 = (T)0;
-#pragma unroll
-                for (int m = 0; m < N; ++m) {
                     du0 = fma(tb.up[j * N + m], fu[m].x, du0);
                     du1 = fma(tb.up[j * N + m], fu[m].y, du1);
                 }
+                // lifts
+                const V2 xf0 = ld2(facep(sXF, 0, j) + 2 * p);
+                const V2 xf1 = ld2(facep(sXF, 1, j) + 2 * p);
+                const V2 xl = xpos ? xf0 : cm0;
+                const V2 xr = xpos ? cmL : xf1;
+                const T tl = vpos ? pa[CONTIG ? -1 : LH - H] : line[0];
+                const T tr = vpos ? line[N - 1] : pa[CONTIG ? N : SL];
+                dx0 = fma(xig0, xl.x, dx0);
+                dx1 = fma(xig0, xl.y, dx1);
+                dv0 = fma(xik00, tl, dv0);
+                dv1 = fma(xik10, tl, dv1);
                 du0 = fma(tb.xi[2 * j], uL0, du0);
-                du0 = fma(-tb.xi[2 * j + 1], uR0, du0);
                 du1 = fma(tb.xi[2 * j], uL1, du1);
+                dx0 = fma(-xig1, xr.x, dx0);
+                dx1 = fma(-xig1, xr.y, dx1);
+                dv0 = fma(-xik01, tr, dv0);
+                dv1 = fma(-xik11, tr, dv1);
+                du0 = fma(-tb.xi[2 * j + 1], uR0, du0);
                 du1 = fma(-tb.xi[2 * j + 1], uR1, du1);
                 T r0 = fma(uxT * dx0, jx, fma(sp0 * du0, ju, (svT * dv0) * jv));
                 T r1 = fma(uxT * dx1, jx, fma(sp1 * du1, ju, (svT * dv1) * jv));
