@@ -716,6 +716,27 @@ int stage_epw(const vl_ctx *c) {
     return 32 / c->cfg.n;
 }
 
+// CTAs per x element of a stage kernel with `slots` resident CTAs on the device.  A CTA walks its
+// tiles one after another and CTAs beyond the resident ones run in further waves, so the time is
+// about waves x (tiles per CTA + a start-up of one tile): the smallest over up to four waves.  (nx = 64
+// elements on 296 slots: 4 CTAs per element leave 40 slots empty in one wave of 352 tiles, 9 fill
+// two waves of 157.)
+int wave_grid(int tiles, int nx, int slots) {
+    int best = 1, best_t = 0, best_waves = 0;
+    for (int g = 1; g <= tiles; ++g) {
+        const int waves = (int)(((int64_t)g * nx + slots - 1) / slots);
+        if (waves > 4 && g > 1) break;
+        const int t = waves * ((tiles + g - 1) / g + 1);
+        // (of equal times with as many waves the larger: more warps in flight)
+        if (g == 1 || t < best_t || (t == best_t && waves == best_waves)) {
+            best_t = t;
+            best_waves = waves;
+            best = g;
+        }
+    }
+    return best;
+}
+
 // ------------------------------------------------------------------------------------------
 // moment kernel dispatch
 // ------------------------------------------------------------------------------------------
@@ -1111,14 +1132,7 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
                         : stage_occupancy<float>(n, c->use_tma, c->use_frag, gen, c->gen_tma, c->gen_pair);
     const int bt = stage_epw(c);
     const int tiles = cfg->nu * ((cfg->nv + bt - 1) / bt);
-    // one wave: at most occ x SMs resident CTAs in total (a second partial wave would double
-    // the kernel time)
-    auto grid_for = [&](int o) {
-        int g = (c->sm_count * o) / cfg->nx;
-        if (g > tiles) g = tiles;
-        if (g < 1) g = 1;
-        return g;
-    };
+    auto grid_for = [&](int o) { return wave_grid(tiles, cfg->nx, c->sm_count * o); };
     c->stage_grid_g = grid_for(occ);
     c->stage_grid_g1 = (c->use_frag && cfg->precision == VL_FP64) ? grid_for(frag_nofn_occupancy())
                                                                   : c->stage_grid_g;

@@ -620,7 +620,8 @@ VL_API int vl_ens_destroy(vl_ens *E) {
 VL_API size_t vl_ens_workspace_bytes(const vl_ens *E, int32_t i) {
     if (!E || i < 0 || i >= (int)E->ctx.size()) return 0;
     const vl_ctx *c = E->ctx[i];
-    return partial_bytes(c, tiles_of(c));   // partials for any schedule
+    // partials for any schedule, and for the context's own stage kernel
+    return partial_bytes(c, std::max(tiles_of(c), std::max(c->stage_grid_g, c->stage_grid_g1)));
 }
 
 VL_API int vl_ens_bind(vl_ens *E, int32_t i, void *f, void *sa, void *sb, double *Ef, double *phi,
