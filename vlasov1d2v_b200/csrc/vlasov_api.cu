@@ -27,6 +27,7 @@
 #include "vlasov_field_conv.cuh"
 #include "vlasov_stage_gen.cuh"
 #include "vlasov_gen_kinds.h"
+#include "vlasov_line.h"
 
 #include "vlasov_ctx.cuh"
 
@@ -543,7 +544,23 @@ int launch_stage(vl_ctx *c, const vl::StageArgs &a, cudaStream_t s) {
     }
 }
 
+// the line-form kernel (vlasov_stage_line.cuh)
+int launch_line(vl_ctx *c, const vl::StageArgs &a0, cudaStream_t s) {
+    vl::StageArgs a = a0;
+    if (a.err == nullptr) a.err = c->d_err;
+    if ((reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.fn) |
+         reinterpret_cast<uintptr_t>(a.ghost_out)) %
+        (uintptr_t)c->state_align)
+        return fail(VL_ERR_INVALID, "state buffers must be " + std::to_string(c->state_align) + "-byte aligned");
+    const vl::LineCoef lc = {c->up, c->xi, c->xw, c->cfg.ju, c->cfg.jv};
+    const dim3 grid(a.kind == vl::KIND_COMBINE ? c->stage_grid_g : c->stage_grid_g1, c->cfg.nx);
+    return check_launch(c->cfg.precision == VL_FP64 ? vl::line_launch<double>(c->cfg.n, a, lc, grid, s)
+                                                    : vl::line_launch<float>(c->cfg.n, a, lc, grid, s),
+                        "stage_line_kernel");
+}
+
 int stage(vl_ctx *c, const vl::StageArgs &a, cudaStream_t s) {
+    if (c->stage_kernel == VL_STAGE_LINE) return launch_line(c, a, s);
     return c->cfg.precision == VL_FP64 ? launch_stage<double>(c, a, s)
                                        : launch_stage<float>(c, a, s);
 }
@@ -1090,13 +1107,19 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
         const char *env = getenv("VLASOV1D2V_NO_FRAG");
         if (env && env[0] == '1') c->use_frag = false;
     }
-    // stage kernel (fastest measured per order and precision): the fragment kernel for n = 8; in
-    // FP64 the generic kernel for every other order (its TMA form where the rows allow); in FP32
-    // the TMA kernel for n = 4, the generic kernel's TMA form on 16-byte rows and the
-    // register-pencil kernel otherwise.
-    // VLASOV1D2V_STAGE_KERNEL=frag|gen|pencil selects one of the forms that apply, for comparisons
-    // FP32 on the generic kernel's TMA form where the rows are 16-byte multiples ((nv+2) n a
-    // multiple of 4), orders other than 4 and 8; VLASOV1D2V_GEN_NO_TMA=1 switches it off
+    // Stage kernel (fastest measured per order and precision):
+    //   n = 8: the fragment kernel (FP64), the packed-FP32 kernel (FP32)
+    //   FP64, other orders: the generic kernel's TMA form where the rows are 16-byte multiples ((nv+2) n
+    //     even); the line form elsewhere (n = 7 at 24x31x33, odd rows: 66 / 90 us per Euler /
+    //     combination stage against 119 / 147 in the generic kernel's cp.async form; on 16-byte rows the
+    //     TMA form is faster: 83 / 89 against 88 / 121 us at 32^3)
+    //   FP32, other orders: the line form (64^3, n = 9: 703 / 865 us against 870 / 912 in the generic
+    //     kernel's paired-row TMA form; n = 7 at 24x31x33 32 / 40 against 56 / 63 in the register-pencil
+    //     kernel; n = 4 at 32x64x64 27 / 32 against 40 / 48 in the order-4 TMA kernel; n = 6 at 32^3
+    //     26.6 / 30.9 against 27.9 / 30.4 in the generic kernel's TMA form)
+    // The line form takes x slabs below 4 GiB (32-bit offsets); beyond, the generic and register-pencil
+    // kernels serve its cases.  VLASOV1D2V_STAGE_KERNEL=frag|gen|pencil|line selects one of the forms
+    // that apply, for comparisons; VLASOV1D2V_GEN_NO_TMA=1 keeps the generic kernel off its TMA forms.
     const bool no_gen_tma = [] {
         const char *env = getenv("VLASOV1D2V_GEN_NO_TMA");
         return env && env[0] == '1';
@@ -1106,11 +1129,19 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
     // FP32 rows of R = 2 mod 4 floats over an even number of rows: the paired-row TMA form
     const bool gen_pair32 = cfg->precision == VL_FP32 && ((size_t)(cfg->nv + 2) * n) % 4 == 2 &&
                             ((size_t)(cfg->nu + 2) * n) % 2 == 0 && !no_gen_tma && encode_fn() != nullptr;
-    c->stage_kernel = c->use_frag                                  ? VL_STAGE_FRAG
-                      : cfg->precision == VL_FP64                  ? VL_STAGE_GEN
-                      : c->use_tma                                 ? VL_STAGE_TMA
-                      : (gen_tma32 || gen_pair32)                  ? VL_STAGE_GEN
-                                                                   : VL_STAGE_PENCIL;
+    const bool line_ok = elems / (size_t)(cfg->nx + 2) * (cfg->precision == VL_FP64 ? 8 : 4) < ((size_t)1 << 32);
+    const bool tma64 = ((size_t)(cfg->nv + 2) * n) % 2 == 0 && encode_fn() != nullptr && !no_gen_tma;
+    // the forms without the line kernel (they also say how the entry points want buffers aligned)
+    const int general = cfg->precision == VL_FP64     ? VL_STAGE_GEN
+                        : c->use_tma                  ? VL_STAGE_TMA
+                        : (gen_tma32 || gen_pair32)   ? VL_STAGE_GEN
+                                                      : VL_STAGE_PENCIL;
+    c->state_align = (cfg->precision == VL_FP64 ? tma64 : general != VL_STAGE_PENCIL) ? 16
+                     : cfg->precision == VL_FP64                                       ? 8
+                                                                                       : 4;
+    c->stage_kernel = c->use_frag                                      ? VL_STAGE_FRAG
+                      : line_ok && !(cfg->precision == VL_FP64 && tma64) ? VL_STAGE_LINE
+                                                                       : general;
     {
         const char *env = getenv("VLASOV1D2V_STAGE_KERNEL");
         if (env) {
@@ -1118,14 +1149,14 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
             if (k == "gen") c->stage_kernel = VL_STAGE_GEN;
             else if (k == "pencil") c->stage_kernel = VL_STAGE_PENCIL;
             else if (k == "frag" && c->use_frag) c->stage_kernel = VL_STAGE_FRAG;
+            else if (k == "line" && line_ok) c->stage_kernel = VL_STAGE_LINE;
         }
         c->use_frag = c->stage_kernel == VL_STAGE_FRAG;
         if (c->stage_kernel != VL_STAGE_TMA && c->stage_kernel != VL_STAGE_FRAG) c->use_tma = false;
     }
     const bool gen = c->stage_kernel == VL_STAGE_GEN;
     // generic kernel in its TMA form: FP64 rows of a 16-byte multiple (V n even), FP32 as above
-    c->gen_tma = gen && (cfg->precision == VL_FP64 ? ((size_t)(cfg->nv + 2) * n) % 2 == 0 : gen_tma32) &&
-                 encode_fn() != nullptr && !no_gen_tma;
+    c->gen_tma = gen && (cfg->precision == VL_FP64 ? tma64 : gen_tma32);
     c->gen_pair = gen && !c->gen_tma && gen_pair32;
     const int occ = cfg->precision == VL_FP64
                         ? stage_occupancy<double>(n, c->use_tma, c->use_frag, gen, c->gen_tma, false)
@@ -1136,6 +1167,14 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
     c->stage_grid_g = grid_for(occ);
     c->stage_grid_g1 = (c->use_frag && cfg->precision == VL_FP64) ? grid_for(frag_nofn_occupancy())
                                                                   : c->stage_grid_g;
+    if (c->stage_kernel == VL_STAGE_LINE) {
+        const bool d = cfg->precision == VL_FP64;
+        auto occ_of = [&](int kind) { return d ? vl::line_occupancy<double>(n, kind) : vl::line_occupancy<float>(n, kind); };
+        const int ept = vl::line_ept(n), lt = cfg->nu * ((cfg->nv + ept - 1) / ept);
+        auto line_grid = [&](int o) { return wave_grid(lt, cfg->nx, c->sm_count * o); };
+        c->stage_grid_g = line_grid(occ_of(vl::KIND_COMBINE));
+        c->stage_grid_g1 = line_grid(std::min(occ_of(vl::KIND_EULER), occ_of(vl::KIND_RHS)));
+    }
     // standalone moment: MOMENT_CTAS_PER_SM resident CTAs per SM, at most one per u element
     int gm = (c->sm_count * vl::MOMENT_CTAS_PER_SM) / cfg->nx;
     if (gm > cfg->nu) gm = cfg->nu;

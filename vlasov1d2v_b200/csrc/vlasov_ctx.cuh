@@ -12,7 +12,7 @@
 #include "vlasov_kernels.cuh"
 #include "vlasov_stage_f32.cuh"
 
-enum vl_stage_kernel { VL_STAGE_PENCIL = 0, VL_STAGE_TMA = 1, VL_STAGE_FRAG = 2, VL_STAGE_GEN = 3 };
+enum vl_stage_kernel { VL_STAGE_PENCIL = 0, VL_STAGE_TMA = 1, VL_STAGE_FRAG = 2, VL_STAGE_GEN = 3, VL_STAGE_LINE = 4 };
 
 struct vl_ctx {
     vl_config cfg;      // scalars (pointer members cleared)
@@ -43,6 +43,7 @@ struct vl_ctx {
     bool use_tma = false;         // stage kernel: TMA-pipelined form (aligned orders)
     bool use_frag = false;        // n = 8: quad-fragment stage kernel (tensor cores in FP64)
     int stage_kernel = VL_STAGE_GEN;   // which stage kernel the launches use (vl_stage_kernel)
+    int state_align = 4;          // alignment that the entry points ask of state buffers (bytes)
     bool gen_tma = false;         // generic stage kernel in its TMA form (FP64, aligned rows)
     bool gen_pair = false;        // generic stage kernel in its paired-row TMA form (FP32, R = 2 mod 4)
     const float *bg_rb = nullptr;   // background-split RHS tables (caller-owned)
