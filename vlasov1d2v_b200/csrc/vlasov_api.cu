@@ -364,6 +364,12 @@ const vl::F32Tables &f32_tables(vl_ctx *c) {
     return c->f32_tables;
 }
 
+// (CTAs per x element, x elements)
+dim3 stage_grid(const vl_ctx *c, const vl::StageArgs &a) {
+    const int g = a.grid_g > 0 ? a.grid_g : a.kind == vl::KIND_COMBINE ? c->stage_grid_g : c->stage_grid_g1;
+    return dim3((unsigned)g, (unsigned)c->cfg.nx);
+}
+
 template <int N, typename T>
 int launch_stage_t(vl_ctx *c, const vl::StageArgs &a0, cudaStream_t s) {
     vl::StageTables<T> tb;
@@ -385,7 +391,7 @@ int launch_stage_t(vl_ctx *c, const vl::StageArgs &a0, cudaStream_t s) {
         }
     vl::StageArgs a = a0;
     if (a.err == nullptr) a.err = c->d_err;
-    dim3 grid(a.kind == vl::KIND_COMBINE ? c->stage_grid_g : c->stage_grid_g1, c->cfg.nx);
+    const dim3 grid = stage_grid(c, a);
     if constexpr (N == 8) {
         if (c->use_frag) {
             using G = vl::FragGeom<T>;
@@ -553,7 +559,7 @@ int launch_line(vl_ctx *c, const vl::StageArgs &a0, cudaStream_t s) {
         (uintptr_t)c->state_align)
         return fail(VL_ERR_INVALID, "state buffers must be " + std::to_string(c->state_align) + "-byte aligned");
     const vl::LineCoef lc = {c->up, c->xi, c->xw, c->cfg.ju, c->cfg.jv};
-    const dim3 grid(a.kind == vl::KIND_COMBINE ? c->stage_grid_g : c->stage_grid_g1, c->cfg.nx);
+    const dim3 grid = stage_grid(c, a);
     return check_launch(c->cfg.precision == VL_FP64 ? vl::line_launch<double>(c->cfg.n, a, lc, grid, s)
                                                     : vl::line_launch<float>(c->cfg.n, a, lc, grid, s),
                         "stage_line_kernel");
@@ -1165,6 +1171,8 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
     const int tiles = cfg->nu * ((cfg->nv + bt - 1) / bt);
     auto grid_for = [&](int o) { return wave_grid(tiles, cfg->nx, c->sm_count * o); };
     c->stage_grid_g = grid_for(occ);
+    c->stage_slots = c->sm_count * occ;
+    c->stage_tiles = tiles;
     c->stage_grid_g1 = (c->use_frag && cfg->precision == VL_FP64) ? grid_for(frag_nofn_occupancy())
                                                                   : c->stage_grid_g;
     if (c->stage_kernel == VL_STAGE_LINE) {
@@ -1172,7 +1180,10 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
         auto occ_of = [&](int kind) { return d ? vl::line_occupancy<double>(n, kind) : vl::line_occupancy<float>(n, kind); };
         const int ept = vl::line_ept(n), lt = cfg->nu * ((cfg->nv + ept - 1) / ept);
         auto line_grid = [&](int o) { return wave_grid(lt, cfg->nx, c->sm_count * o); };
-        c->stage_grid_g = line_grid(occ_of(vl::KIND_COMBINE));
+        const int lo = occ_of(vl::KIND_COMBINE);
+        c->stage_grid_g = line_grid(lo);
+        c->stage_slots = c->sm_count * lo;
+        c->stage_tiles = lt;
         c->stage_grid_g1 = line_grid(std::min(occ_of(vl::KIND_EULER), occ_of(vl::KIND_RHS)));
     }
     // standalone moment: MOMENT_CTAS_PER_SM resident CTAs per SM, at most one per u element

@@ -72,6 +72,7 @@ struct StageArgs {
     // context's Jacobians; a call with other direction weights (jx, jv above) scales them by
     // jx / J_x and jv / J_v (the RHS kind only; the RK stages use the context's Jacobians)
     double sx, sv;
+    int grid_g;  // CTAs per x element (0: the context's own choice; host side)
     int never;   // line-form kernel: a value that no tile index takes (-1)
 };
 
