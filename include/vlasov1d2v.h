@@ -318,10 +318,10 @@ VL_API int vl_mlp_dims(int32_t *in, int32_t *hidden, int32_t *out, int32_t *n_we
  * vl_mlp_backward (all three or none).                                                      */
 VL_API int vl_mlp_forward(const float *X, int32_t nrows, const void *wf, const void *wb, const float *bias,
                           float *Y, void *H0, void *Hh, float *Z, void *stream);
-/* FP32 elements of the per-block gradient partials vl_mlp_backward needs for nrows samples. */
+/* FP32 elements of the scratch vl_mlp_backward needs for nrows samples (`partials`).          */
 VL_API size_t vl_mlp_partial_floats(int32_t nrows);
 /* Gradient of L = sum_{rows, c < nout} (Y - T)^2 / (nrows nout), T[nrows][nout], through the
- * network (bf16 operands, FP32 accumulation; per-block partials summed in a fixed order):
+ * network (bf16 operands, FP32 accumulation; blocks of 64 samples summed in a fixed order):
  * grad_w in the [in][out] layout, grad_b.                                                    */
 VL_API int vl_mlp_backward(const float *Y, const float *T, int32_t nrows, int32_t nout, const void *wf,
                            const void *wb, const float *bias, const void *H0, const void *Hh, const float *Z,

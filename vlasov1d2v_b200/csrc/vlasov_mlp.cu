@@ -3,17 +3,20 @@
 // training-forward, backward, gradient-reduction and Adam kernels, plus the closure's feature
 // extraction from a coarse state and the application of its correction to an RK stage.
 //
-// Matrix products run on the tensor cores with mma.sync.m16n8k16 (bf16 x bf16 -> f32).  A warp
-// owns 16 samples; the accumulator fragment of one layer (rows g, g + 8; columns 2t, 2t + 1 of
-// each 8-column tile, g = lane / 4, t = lane % 4) is exactly the A fragment of the next layer's
-// 16-column k tiles, so the activations of a sample tile stay in registers through the network.
-// Weights are read as 32-bit pairs from two layouts kept by the optimizer: [out][in] for the
-// forward product and [in][out] for the backward product.  The weight-gradient product
-// (H^T dZ, a reduction over samples) goes through shared memory.
+// Matrix products run on the tensor cores with mma.sync.m16n8k16 (bf16 x bf16 -> f32).  The forward
+// and the backpropagation kernels give a CTA 32 samples and split a layer's output columns over its 8
+// warps: activations pass from layer to layer through shared memory (ldmatrix), where the next layer's
+// weights arrive by cp.async meanwhile, from the two layouts kept by the optimizer ([out][in] forward,
+// [in][out] backward).  The weight gradients H^T dZ are one kernel over output tiles (mlp_grad_kernel).
+// At minibatches of this size all three are bound by the latency of their chains (layers, summation
+// blocks), not by a rate.  Minibatch of 8192: forward 14 us (28.9 with one warp per 16 samples carrying the
+// whole network in its registers), backward 51 us (110 with the gradients of every 64 samples written as
+// a partial and reduced); of 576: 9 and 17 us (28 and 97).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 
 #include "vlasov1d2v.h"
@@ -24,7 +27,8 @@ namespace {
 
 constexpr int IN = 96, HID = 128, OUT = 48;
 constexpr int NL = 4;                          // layers
-constexpr int WARPS = 4, ROWS = 16 * WARPS;    // samples per CTA tile
+constexpr int WARPS = 8, ROWS = 32;            // warps and samples per CTA (forward, backpropagation)
+constexpr int BLOCK = 64;                      // samples per summation block of the gradients
 __host__ __device__ constexpr int layer_in(int l) { return l == 0 ? IN : HID; }
 __host__ __device__ constexpr int layer_out(int l) { return l == NL - 1 ? OUT : HID; }
 
@@ -55,292 +59,376 @@ __device__ __forceinline__ float gelu_d(float x) {
     return cdf + x * pdf;
 }
 
-// A fragments (bf16 pairs) of a 16 x K row tile from FP32 accumulator fragments of K/8 n tiles:
-// k tile kk takes n tiles 2kk (a0, a1) and 2kk + 1 (a2, a3)
-template <int K>
-__device__ __forceinline__ void acc_to_a(const float (&acc)[K / 8][4], uint32_t (&a)[K / 16][4]) {
-#pragma unroll
-    for (int kk = 0; kk < K / 16; ++kk) {
-        a[kk][0] = pack_bf16(acc[2 * kk][0], acc[2 * kk][1]);
-        a[kk][1] = pack_bf16(acc[2 * kk][2], acc[2 * kk][3]);
-        a[kk][2] = pack_bf16(acc[2 * kk + 1][0], acc[2 * kk + 1][1]);
-        a[kk][3] = pack_bf16(acc[2 * kk + 1][2], acc[2 * kk + 1][3]);
-    }
+// shared-memory row stride (bf16) of a K-wide activation tile: an odd number of 16-byte units, so the
+// eight rows of an ldmatrix fall in distinct banks
+__host__ __device__ constexpr int act_stride(int K) { return K + 8; }
+
+__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const __nv_bfloat16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const __nv_bfloat16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
 
-// acc[n tile][4] = A (16 x K, fragments) . W (K x N), W given as wf[N][K] (bf16)
+__device__ __forceinline__ void cp16(void *dst, const void *src, bool in = true) {   // (zeros when !in)
+    const int bytes = in ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes)
+                 : "memory");
+}
+
+// a layer's weights [N][K] (bf16) to shared memory, rows of act_stride(K)
 template <int K, int N>
-__device__ __forceinline__ void layer_mma(const uint32_t (&a)[K / 16][4], const __nv_bfloat16 *__restrict__ wf,
-                                          float (&acc)[N / 8][4], int g, int t) {
-#pragma unroll
-    for (int nn = 0; nn < N / 8; ++nn) {
-        acc[nn][0] = acc[nn][1] = acc[nn][2] = acc[nn][3] = 0.0f;
-        const uint32_t *wr = reinterpret_cast<const uint32_t *>(wf + (size_t)(8 * nn + g) * K);
-#pragma unroll
-        for (int kk = 0; kk < K / 16; ++kk) {
-            const uint32_t b0 = __ldg(wr + 8 * kk + t);       // k = 16 kk + 2t, +1
-            const uint32_t b1 = __ldg(wr + 8 * kk + 4 + t);   // k = 16 kk + 8 + 2t, +1
-            mma_bf16(acc[nn], a[kk], b0, b1);
+__device__ __forceinline__ void stage_weights(__nv_bfloat16 *sW, const __nv_bfloat16 *__restrict__ w) {
+    if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+        for (int q = threadIdx.x; q < N * K / 8; q += 32 * WARPS) {
+            const int n = q / (K / 8), c = 8 * (q - n * (K / 8));
+            cp16(sW + n * act_stride(K) + c, w + n * K + c);
+        }
+    } else {   // not on a 16-byte boundary: pairs
+        for (int q = threadIdx.x; q < N * K / 2; q += 32 * WARPS) {
+            const int n = q / (K / 2), c = 2 * (q - n * (K / 2));
+            *reinterpret_cast<uint32_t *>(sW + n * act_stride(K) + c) =
+                __ldg(reinterpret_cast<const uint32_t *>(w + n * K + c));
         }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int LEFT>
+__device__ __forceinline__ void weights_ready() {   // all but the last LEFT staged layers, and the activations
+    asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+    __syncthreads();
 }
 
-template <int N>
-__device__ __forceinline__ void add_bias(float (&acc)[N / 8][4], const float *__restrict__ bias, int t) {
+// acc[row tile][column tile][4] = A (the CTA's ROWS x K activations) . the warp's weight columns
+template <int K, int NT>
+__device__ __forceinline__ void layer_mma(const __nv_bfloat16 *sA, const __nv_bfloat16 *sW, int n0, int lane,
+                                          float (&acc)[ROWS / 16][NT][4]) {
+    const __nv_bfloat16 *pw = sW + (8 * n0 + (lane & 7)) * act_stride(K) + (lane >> 3) * 8;
+    uint32_t b[NT][4];   // two k tiles of each column tile
+    const __nv_bfloat16 *p = sA + ((lane & 7) + ((lane >> 3) & 1) * 8) * act_stride(K) + (lane >> 4) * 8;
 #pragma unroll
-    for (int nn = 0; nn < N / 8; ++nn) {
-        const float b0 = __ldg(bias + 8 * nn + 2 * t), b1 = __ldg(bias + 8 * nn + 2 * t + 1);
-        acc[nn][0] += b0;
-        acc[nn][1] += b1;
-        acc[nn][2] += b0;
-        acc[nn][3] += b1;
-    }
-}
-
-// input A fragments of a 16-row tile of X [rows][IN] (FP32 in memory, rounded to bf16)
-__device__ __forceinline__ void load_input(const float *__restrict__ X, int row0, int nrows, int g, int t,
-                                           uint32_t (&a)[IN / 16][4]) {
-    const int r0 = row0 + g, r1 = row0 + g + 8;
+    for (int mm = 0; mm < ROWS / 16; ++mm)
 #pragma unroll
-    for (int kk = 0; kk < IN / 16; ++kk) {
-        const int c = 16 * kk + 2 * t;
-        float2 v00 = make_float2(0.f, 0.f), v10 = v00, v01 = v00, v11 = v00;
-        if (r0 < nrows) {
-            v00 = *reinterpret_cast<const float2 *>(X + (size_t)r0 * IN + c);
-            v01 = *reinterpret_cast<const float2 *>(X + (size_t)r0 * IN + c + 8);
-        }
-        if (r1 < nrows) {
-            v10 = *reinterpret_cast<const float2 *>(X + (size_t)r1 * IN + c);
-            v11 = *reinterpret_cast<const float2 *>(X + (size_t)r1 * IN + c + 8);
-        }
-        a[kk][0] = pack_bf16(v00.x, v00.y);
-        a[kk][1] = pack_bf16(v10.x, v10.y);
-        a[kk][2] = pack_bf16(v01.x, v01.y);
-        a[kk][3] = pack_bf16(v11.x, v11.y);
-    }
-}
-
-// store accumulator fragments [16 rows x N] as FP32 rows (stride ld)
-template <int N>
-__device__ __forceinline__ void store_acc(float *__restrict__ Y, int ld, int row0, int nrows, int g, int t,
-                                          const float (&acc)[N / 8][4]) {
-    const int r0 = row0 + g, r1 = row0 + g + 8;
-#pragma unroll
-    for (int nn = 0; nn < N / 8; ++nn) {
-        const int c = 8 * nn + 2 * t;
-        if (r0 < nrows) *reinterpret_cast<float2 *>(Y + (size_t)r0 * ld + c) = make_float2(acc[nn][0], acc[nn][1]);
-        if (r1 < nrows) *reinterpret_cast<float2 *>(Y + (size_t)r1 * ld + c) = make_float2(acc[nn][2], acc[nn][3]);
-    }
-}
-
-// bf16 A-fragment tile [16 rows x K] as rows (stride K)
-template <int K>
-__device__ __forceinline__ void store_a(__nv_bfloat16 *__restrict__ H, int row0, int nrows, int g, int t,
-                                        const uint32_t (&a)[K / 16][4]) {
-    const int r0 = row0 + g, r1 = row0 + g + 8;
-    uint32_t *h = reinterpret_cast<uint32_t *>(H);
+        for (int nn = 0; nn < NT; ++nn) acc[mm][nn][0] = acc[mm][nn][1] = acc[mm][nn][2] = acc[mm][nn][3] = 0.0f;
 #pragma unroll
     for (int kk = 0; kk < K / 16; ++kk) {
-        const int c = 16 * kk + 2 * t;
-        if (r0 < nrows) {
-            h[((size_t)r0 * K + c) / 2] = a[kk][0];
-            h[((size_t)r0 * K + c + 8) / 2] = a[kk][2];
-        }
-        if (r1 < nrows) {
-            h[((size_t)r1 * K + c) / 2] = a[kk][1];
-            h[((size_t)r1 * K + c + 8) / 2] = a[kk][3];
-        }
-    }
-}
-
-template <int K>
-__device__ __forceinline__ void load_a(const __nv_bfloat16 *__restrict__ H, int row0, int nrows, int g, int t,
-                                       uint32_t (&a)[K / 16][4]) {
-    const int r0 = row0 + g, r1 = row0 + g + 8;
-    const uint32_t *h = reinterpret_cast<const uint32_t *>(H);
+        if (kk % 2 == 0) {   // (the last k tile of an odd count: its own columns again as the second half)
 #pragma unroll
-    for (int kk = 0; kk < K / 16; ++kk) {
-        const int c = 16 * kk + 2 * t;
-        a[kk][0] = r0 < nrows ? h[((size_t)r0 * K + c) / 2] : 0u;
-        a[kk][2] = r0 < nrows ? h[((size_t)r0 * K + c + 8) / 2] : 0u;
-        a[kk][1] = r1 < nrows ? h[((size_t)r1 * K + c) / 2] : 0u;
-        a[kk][3] = r1 < nrows ? h[((size_t)r1 * K + c + 8) / 2] : 0u;
+            for (int nn = 0; nn < NT; ++nn) {
+                if (kk + 1 < K / 16)
+                    ldsm_x4(b[nn], pw + 8 * nn * act_stride(K) + 16 * kk);
+                else
+                    ldsm_x4(b[nn], pw + 8 * nn * act_stride(K) + 16 * kk - (lane >> 4) * 16);
+            }
+        }
+#pragma unroll
+        for (int mm = 0; mm < ROWS / 16; ++mm) {
+            uint32_t a[4];
+            ldsm_x4(a, p + mm * 16 * act_stride(K) + 16 * kk);
+#pragma unroll
+            for (int nn = 0; nn < NT; ++nn) mma_bf16(acc[mm][nn], a, b[nn][2 * (kk & 1)], b[nn][2 * (kk & 1) + 1]);
+        }
     }
 }
 
+// dynamic shared memory of the two kernels: two activation tiles, two layers' weights (bf16 elements)
+constexpr int SMEM_A = ROWS * act_stride(HID), SMEM_W = HID * act_stride(HID);
+constexpr int MLP_SMEM = (2 * SMEM_A + 2 * SMEM_W) * (int)sizeof(__nv_bfloat16);
+
 // ---------------------------------------------------------------------------------------------
-// forward: Y = MLP(X); with save != 0 also H_l (bf16 layer inputs) and Z_l (FP32 hidden
-// pre-activations) for the backward pass.  One warp per 16-sample tile, grid-stride over tiles.
+// forward: Y = MLP(X); with H0 also H_l (bf16 layer inputs) and Z_l (FP32 hidden pre-activations) for
+// the backward pass.  One CTA per ROWS samples.
 // ---------------------------------------------------------------------------------------------
+// one hidden layer: bias, pre-activation out, GELU, bf16 activation to the next tile (and out)
+template <int K>
+__device__ __forceinline__ void forward_hidden(const __nv_bfloat16 *sA, const __nv_bfloat16 *sW,
+                                               const float *__restrict__ bias, int n0, int row0, int nrows, int lane,
+                                               float *__restrict__ Z, __nv_bfloat16 *__restrict__ H,
+                                               __nv_bfloat16 *sNext) {
+    const int g = lane >> 2, t = lane & 3;
+    float acc[ROWS / 16][2][4];
+    layer_mma<K, 2>(sA, sW, n0, lane, acc);
+#pragma unroll
+    for (int nn = 0; nn < 2; ++nn) {
+        const int c = 8 * (n0 + nn) + 2 * t;
+        const float b0 = __ldg(bias + c), b1 = __ldg(bias + c + 1);
+#pragma unroll
+        for (int mm = 0; mm < ROWS / 16; ++mm)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = 16 * mm + 8 * h + g, row = row0 + r;
+                const float z0 = acc[mm][nn][2 * h] + b0, z1 = acc[mm][nn][2 * h + 1] + b1;
+                const uint32_t hv = pack_bf16(gelu(z0), gelu(z1));
+                *reinterpret_cast<uint32_t *>(sNext + r * act_stride(HID) + c) = hv;
+                if (Z != nullptr && row < nrows) {
+                    *reinterpret_cast<float2 *>(Z + (size_t)row * HID + c) = make_float2(z0, z1);
+                    *reinterpret_cast<uint32_t *>(H + (size_t)row * HID + c) = hv;
+                }
+            }
+    }
+}
+
 __global__ void __launch_bounds__(32 * WARPS) mlp_forward_kernel(const float *__restrict__ X, int nrows,
                                                                   MlpWeights w, float *__restrict__ Y,
                                                                   __nv_bfloat16 *__restrict__ H0,
                                                                   __nv_bfloat16 *__restrict__ Hh,
                                                                   float *__restrict__ Z) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int ntile = (nrows + 15) / 16;
-    for (int tile = blockIdx.x * WARPS + (threadIdx.x >> 5); tile < ntile; tile += gridDim.x * WARPS) {
-        const int row0 = tile * 16;
-        uint32_t a0[IN / 16][4];
-        load_input(X, row0, nrows, g, t, a0);
-        if (H0) store_a<IN>(H0, row0, nrows, g, t, a0);
-        float acc[HID / 8][4];
-        layer_mma<IN, HID>(a0, w.wf[0], acc, g, t);
-        add_bias<HID>(acc, w.bias[0], t);
-        uint32_t ah[HID / 16][4];
-#pragma unroll
-        for (int l = 1; l < NL; ++l) {
-            if (Z) store_acc<HID>(Z + (size_t)(l - 1) * nrows * HID, HID, row0, nrows, g, t, acc);
-#pragma unroll
-            for (int nn = 0; nn < HID / 8; ++nn)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) acc[nn][q] = gelu(acc[nn][q]);
-            acc_to_a<HID>(acc, ah);
-            if (Hh) store_a<HID>(Hh + (size_t)(l - 1) * nrows * HID, row0, nrows, g, t, ah);
-            if (l < NL - 1) {
-                layer_mma<HID, HID>(ah, w.wf[l], acc, g, t);
-                add_bias<HID>(acc, w.bias[l], t);
-            }
+    extern __shared__ __align__(16) __nv_bfloat16 mlp_smem[];
+    __nv_bfloat16 *sA[2] = {mlp_smem, mlp_smem + SMEM_A}, *sW[2] = {mlp_smem + 2 * SMEM_A, mlp_smem + 2 * SMEM_A + SMEM_W};
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int row0 = blockIdx.x * ROWS;
+    stage_weights<IN, HID>(sW[0], w.wf[0]);
+    stage_weights<HID, HID>(sW[1], w.wf[1]);
+    for (int q = tid; q < ROWS * IN / 2; q += 32 * WARPS) {   // input, rounded to bf16
+        const int r = q / (IN / 2), c = 2 * (q - r * (IN / 2)), row = row0 + r;
+        uint32_t v = 0u;
+        if (row < nrows) {
+            const float2 x = *reinterpret_cast<const float2 *>(X + (size_t)row * IN + c);
+            v = pack_bf16(x.x, x.y);
+            if (H0) *reinterpret_cast<uint32_t *>(H0 + (size_t)row * IN + c) = v;
         }
-        float out[OUT / 8][4];
-        layer_mma<HID, OUT>(ah, w.wf[NL - 1], out, g, t);
-        add_bias<OUT>(out, w.bias[NL - 1], t);
-        store_acc<OUT>(Y, OUT, row0, nrows, g, t, out);
+        *reinterpret_cast<uint32_t *>(&sA[0][r * act_stride(IN) + c]) = v;
+    }
+    const size_t hs = (size_t)nrows * HID;
+    weights_ready<1>();
+    forward_hidden<IN>(sA[0], sW[0], w.bias[0], 2 * wp, row0, nrows, lane, Z, Hh, sA[1]);
+    weights_ready<0>();
+    stage_weights<HID, HID>(sW[0], w.wf[2]);
+    forward_hidden<HID>(sA[1], sW[1], w.bias[1], 2 * wp, row0, nrows, lane, Z ? Z + hs : nullptr, Hh + hs, sA[0]);
+    weights_ready<0>();
+    stage_weights<HID, OUT>(sW[1], w.wf[NL - 1]);
+    forward_hidden<HID>(sA[0], sW[0], w.bias[2], 2 * wp, row0, nrows, lane, Z ? Z + 2 * hs : nullptr, Hh + 2 * hs, sA[1]);
+    weights_ready<0>();
+    if (wp < OUT / 8) {
+        float acc[ROWS / 16][1][4];
+        layer_mma<HID, 1>(sA[1], sW[1], wp, lane, acc);
+        const int c = 8 * wp + 2 * t;
+        const float y0 = __ldg(w.bias[NL - 1] + c), y1 = __ldg(w.bias[NL - 1] + c + 1);
+#pragma unroll
+        for (int mm = 0; mm < ROWS / 16; ++mm)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int row = row0 + 16 * mm + 8 * h + g;
+                if (row < nrows)
+                    *reinterpret_cast<float2 *>(Y + (size_t)row * OUT + c) =
+                        make_float2(acc[mm][0][2 * h] + y0, acc[mm][0][2 * h + 1] + y1);
+            }
     }
 }
 
 // ---------------------------------------------------------------------------------------------
 // backward of the mean-squared loss over the first nout outputs:
 //   L = sum_rows sum_{c < nout} (Y - T)^2 / (nrows nout)
-// One CTA per 64-sample block: dZ fragments flow back through the layers in registers
-// (dH = dZ W^T, dZ = dH * GELU'(Z)); the weight gradient of each layer, H^T dZ over the block's
-// samples, is formed from shared-memory copies of H and dZ and written as the block's partial
-// (reduced across blocks by mlp_reduce_kernel).
+// mlp_backprop_kernel: dZ of every layer (dH = dZ W^T, dZ = dH * GELU'(Z)), bf16, zero rows up to a
+// multiple of BLOCK samples.  mlp_grad_kernel: gW_l = H_l^T dZ_l and gb_l = sum of dZ_l.
 // ---------------------------------------------------------------------------------------------
 constexpr int GW_ELEMS = IN * HID + 2 * HID * HID + HID * OUT;   // weight elements
 constexpr int GB_ELEMS = 3 * HID + OUT;                          // bias elements
 __host__ __device__ constexpr int w_off(int l) { return l == 0 ? 0 : IN * HID + (l - 1) * HID * HID; }
 __host__ __device__ constexpr int b_off(int l) { return l * HID; }
 
-template <int K, int N>
-__device__ void block_wgrad(const __nv_bfloat16 *sH, const __nv_bfloat16 *sD, float *gw, float *gb) {
-    // gw[k][n] = sum_r sH[r][k] sD[r][n] over ROWS samples; warp w takes n tiles w, w + 4, ...
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, w = threadIdx.x >> 5;
-    for (int nn = w; nn < N / 8; nn += WARPS) {
-        for (int mm = 0; mm < K / 16; ++mm) {
-            float d[4] = {0.f, 0.f, 0.f, 0.f};
+// dZ buffers, back to back: three hidden layers [rows][HID], then the output layer [rows][OUT]
+__host__ __device__ constexpr size_t dz_off(int l, size_t rows) { return (size_t)l * rows * HID; }
+
+// dZ of a hidden layer from the next layer's dZ (sD, K wide): W^T given as wb [HID][K]
+template <int K>
+__device__ __forceinline__ void backprop_hidden(const __nv_bfloat16 *sD, const __nv_bfloat16 *sW,
+                                                const float *__restrict__ Z, int n0, int row0, int nrows, int lane,
+                                                __nv_bfloat16 *__restrict__ dZ, __nv_bfloat16 *sNext) {
+    const int g = lane >> 2, t = lane & 3;
+    float acc[ROWS / 16][2][4];
+    layer_mma<K, 2>(sD, sW, n0, lane, acc);
 #pragma unroll
-            for (int kk = 0; kk < ROWS / 16; ++kk) {
-                // A = H^T (16 k-rows of weight index x 16 samples), B = dZ (16 samples x 8 outputs)
-                const int r = 16 * kk + 2 * t;
-                const int m0 = 16 * mm + g, m1 = m0 + 8;
-                uint32_t a[4];
-                a[0] = pack_bf16(__bfloat162float(sH[r * K + m0]), __bfloat162float(sH[(r + 1) * K + m0]));
-                a[1] = pack_bf16(__bfloat162float(sH[r * K + m1]), __bfloat162float(sH[(r + 1) * K + m1]));
-                a[2] = pack_bf16(__bfloat162float(sH[(r + 8) * K + m0]), __bfloat162float(sH[(r + 9) * K + m0]));
-                a[3] = pack_bf16(__bfloat162float(sH[(r + 8) * K + m1]), __bfloat162float(sH[(r + 9) * K + m1]));
-                const int n = 8 * nn + g;
-                const uint32_t b0 = pack_bf16(__bfloat162float(sD[r * N + n]), __bfloat162float(sD[(r + 1) * N + n]));
-                const uint32_t b1 = pack_bf16(__bfloat162float(sD[(r + 8) * N + n]), __bfloat162float(sD[(r + 9) * N + n]));
-                mma_bf16(d, a, b0, b1);
+    for (int nn = 0; nn < 2; ++nn) {
+        const int c = 8 * (n0 + nn) + 2 * t;
+#pragma unroll
+        for (int mm = 0; mm < ROWS / 16; ++mm)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = 16 * mm + 8 * h + g, row = row0 + r;
+                float d0 = 0.f, d1 = 0.f;
+                if (row < nrows) {
+                    const float2 z = *reinterpret_cast<const float2 *>(Z + (size_t)row * HID + c);
+                    d0 = acc[mm][nn][2 * h] * gelu_d(z.x);
+                    d1 = acc[mm][nn][2 * h + 1] * gelu_d(z.y);
+                }
+                const uint32_t v = pack_bf16(d0, d1);
+                *reinterpret_cast<uint32_t *>(dZ + (size_t)row * HID + c) = v;
+                *reinterpret_cast<uint32_t *>(sNext + r * act_stride(HID) + c) = v;
             }
-            const int m0 = 16 * mm + g, c = 8 * nn + 2 * t;
-            gw[(size_t)m0 * N + c] = d[0];
-            gw[(size_t)m0 * N + c + 1] = d[1];
-            gw[(size_t)(m0 + 8) * N + c] = d[2];
-            gw[(size_t)(m0 + 8) * N + c + 1] = d[3];
-        }
-    }
-    // bias gradient: column sums of dZ (FP32 from the bf16 copy)
-    for (int n = threadIdx.x; n < N; n += blockDim.x) {
-        float s = 0.f;
-        for (int r = 0; r < ROWS; ++r) s += __bfloat162float(sD[r * N + n]);
-        gb[n] = s;
     }
 }
 
-__global__ void __launch_bounds__(32 * WARPS) mlp_backward_kernel(const float *__restrict__ Y,
-                                                                   const float *__restrict__ T, int nrows,
-                                                                   int nout, MlpWeights w,
-                                                                   const __nv_bfloat16 *__restrict__ H0,
-                                                                   const __nv_bfloat16 *__restrict__ Hh,
-                                                                   const float *__restrict__ Z,
-                                                                   float *__restrict__ gw_part,
-                                                                   float *__restrict__ gb_part) {
-    __shared__ __align__(16) __nv_bfloat16 sH[ROWS * HID];
-    __shared__ __align__(16) __nv_bfloat16 sD[ROWS * HID];
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, wp = threadIdx.x >> 5;
-    const int row0 = blockIdx.x * ROWS + 16 * wp;
-    const int r0 = row0 + g, r1 = row0 + g + 8;
-    float *gw = gw_part + (size_t)blockIdx.x * GW_ELEMS;
-    float *gb = gb_part + (size_t)blockIdx.x * GB_ELEMS;
+__global__ void __launch_bounds__(32 * WARPS) mlp_backprop_kernel(const float *__restrict__ Y,
+                                                                   const float *__restrict__ T, int nrows, int nout,
+                                                                   MlpWeights w, const float *__restrict__ Z,
+                                                                   __nv_bfloat16 *__restrict__ dZ, int rows) {
+    extern __shared__ __align__(16) __nv_bfloat16 mlp_smem[];
+    __nv_bfloat16 *sD[2] = {mlp_smem, mlp_smem + SMEM_A}, *sW[2] = {mlp_smem + 2 * SMEM_A, mlp_smem + 2 * SMEM_A + SMEM_W};
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    const int row0 = blockIdx.x * ROWS;
+    stage_weights<OUT, HID>(sW[0], w.wb[NL - 1]);
+    stage_weights<HID, HID>(sW[1], w.wb[2]);
     const float scale = 2.0f / ((float)nrows * (float)nout);
-    // dZ of the output layer (linear): dL/dY
-    float dz[OUT / 8][4];
-#pragma unroll
-    for (int nn = 0; nn < OUT / 8; ++nn)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int r = (q < 2) ? r0 : r1, c = 8 * nn + 2 * t + (q & 1);
-            float v = 0.f;
-            if (r < nrows && c < nout) v = scale * (Y[(size_t)r * OUT + c] - T[(size_t)r * nout + c]);
-            dz[nn][q] = v;
+    for (int q = tid; q < ROWS * OUT / 2; q += 32 * WARPS) {   // dZ of the output layer (linear): dL/dY
+        const int r = q / (OUT / 2), c = 2 * (q - r * (OUT / 2)), row = row0 + r;
+        float v0 = 0.f, v1 = 0.f;
+        if (row < nrows) {
+            if (c < nout) v0 = scale * (Y[(size_t)row * OUT + c] - T[(size_t)row * nout + c]);
+            if (c + 1 < nout) v1 = scale * (Y[(size_t)row * OUT + c + 1] - T[(size_t)row * nout + c + 1]);
         }
-    uint32_t adz[OUT / 16][4];
-    acc_to_a<OUT>(dz, adz);
-    // ---- layer NL-1 (HID -> OUT) ----
-    {
-        uint32_t ah[HID / 16][4];
-        load_a<HID>(Hh + (size_t)(NL - 2) * nrows * HID, row0, nrows, g, t, ah);
-        store_a<HID>(sH, 16 * wp, ROWS, g, t, ah);
-        store_a<OUT>(sD, 16 * wp, ROWS, g, t, adz);
-        __syncthreads();
-        block_wgrad<HID, OUT>(sH, sD, gw + w_off(NL - 1), gb + b_off(NL - 1));
-        __syncthreads();
+        const uint32_t v = pack_bf16(v0, v1);
+        *reinterpret_cast<uint32_t *>(&sD[0][r * act_stride(OUT) + c]) = v;
+        *reinterpret_cast<uint32_t *>(dZ + dz_off(NL - 1, rows) + (size_t)row * OUT + c) = v;
     }
-    // dH = dZ W^T: W^T given by wb[in][out] rows (in = output index n of this product)
-    float dh[HID / 8][4];
-    layer_mma<OUT, HID>(adz, w.wb[NL - 1], dh, g, t);
-    for (int l = NL - 2; l >= 0; --l) {
-        // dZ_l = dH * GELU'(Z_l)
-        const float *Zl = Z + (size_t)l * nrows * HID;
-#pragma unroll
-        for (int nn = 0; nn < HID / 8; ++nn)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = (q < 2) ? r0 : r1, c = 8 * nn + 2 * t + (q & 1);
-                dh[nn][q] = (r < nrows) ? dh[nn][q] * gelu_d(Zl[(size_t)r * HID + c]) : 0.f;
-            }
-        uint32_t ad[HID / 16][4];
-        acc_to_a<HID>(dh, ad);
-        const int K = layer_in(l);
-        if (l == 0) {
-            uint32_t ah[IN / 16][4];
-            load_a<IN>(H0, row0, nrows, g, t, ah);
-            store_a<IN>(sH, 16 * wp, ROWS, g, t, ah);
-        } else {
-            uint32_t ah[HID / 16][4];
-            load_a<HID>(Hh + (size_t)(l - 1) * nrows * HID, row0, nrows, g, t, ah);
-            store_a<HID>(sH, 16 * wp, ROWS, g, t, ah);
-        }
-        store_a<HID>(sD, 16 * wp, ROWS, g, t, ad);
-        __syncthreads();
-        if (K == IN)
-            block_wgrad<IN, HID>(sH, sD, gw + w_off(l), gb + b_off(l));
-        else
-            block_wgrad<HID, HID>(sH, sD, gw + w_off(l), gb + b_off(l));
-        __syncthreads();
-        if (l > 0) layer_mma<HID, HID>(ad, w.wb[l], dh, g, t);
-    }
+    const size_t hs = (size_t)nrows * HID;
+    weights_ready<1>();
+    backprop_hidden<OUT>(sD[0], sW[0], Z + 2 * hs, 2 * wp, row0, nrows, lane, dZ + dz_off(2, rows), sD[1]);
+    weights_ready<0>();
+    stage_weights<HID, HID>(sW[0], w.wb[1]);
+    backprop_hidden<HID>(sD[1], sW[1], Z + hs, 2 * wp, row0, nrows, lane, dZ + dz_off(1, rows), sD[0]);
+    weights_ready<0>();
+    backprop_hidden<HID>(sD[0], sW[0], Z, 2 * wp, row0, nrows, lane, dZ + dz_off(0, rows), sD[1]);
 }
 
-// sum the per-block partial gradients (fixed order: deterministic)
-__global__ void mlp_reduce_kernel(const float *__restrict__ part, int nblocks, int n, float *__restrict__ out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int b = 0; b < nblocks; ++b) s += part[(size_t)b * n + i];
-        out[i] = s;
+// Gradients.  CTA < GRAD_TILES: a 16 x 32 tile of one layer's gW (warp: 16 x 8) over all samples, which
+// stream through shared memory 256 at a time; a block of BLOCK samples is one chain of four MMAs, added
+// to the running FP32 sum in the order of the blocks.  The other CTAs: four columns of gb, one thread
+// per block of samples, then their sums in order.  No partial gradients in memory (26 MB written and read
+// back per minibatch of 8192 with one partial per block).
+constexpr int GM = 16, GN = 32, GCH = 4 * BLOCK, GST = 3;   // tile, samples per stage, stages
+constexpr int SHS = GM + 8, SDS = GN + 8;                   // row strides: 48 and 80 bytes, conflict-free
+constexpr int GRAD_THREADS = 128;
+constexpr int GRAD_SMEM = GST * GCH * (SHS + SDS) * (int)sizeof(__nv_bfloat16);
+__host__ __device__ constexpr int grad_ngroups(int l) { return (layer_out(l) + GN - 1) / GN; }
+__host__ __device__ constexpr int grad_tiles(int l) { return layer_in(l) / GM * grad_ngroups(l); }
+constexpr int GRAD_TILES = grad_tiles(0) + grad_tiles(1) + grad_tiles(2) + grad_tiles(3);
+constexpr int BIAS_CTAS = GB_ELEMS / 4;
+
+__global__ void __launch_bounds__(GRAD_THREADS) mlp_grad_kernel(const __nv_bfloat16 *__restrict__ H0,
+                                                                 const __nv_bfloat16 *__restrict__ Hh,
+                                                                 const __nv_bfloat16 *__restrict__ dZ, int nrows,
+                                                                 int rows, bool h16, float *__restrict__ grad_w,
+                                                                 float *__restrict__ grad_b) {
+    extern __shared__ __align__(16) __nv_bfloat16 mlp_smem[];
+    __nv_bfloat16(*sH)[GCH * SHS] = reinterpret_cast<__nv_bfloat16(*)[GCH * SHS]>(mlp_smem);
+    __nv_bfloat16(*sD)[GCH * SDS] = reinterpret_cast<__nv_bfloat16(*)[GCH * SDS]>(mlp_smem + GST * GCH * SHS);
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    if (blockIdx.x >= GRAD_TILES) {
+        // bias columns [c, c + 4) of layer l
+        int c = (blockIdx.x - GRAD_TILES) * 4, l = 0;
+        while (l < NL - 1 && c >= b_off(l + 1)) ++l;
+        const int N = layer_out(l), n = c - b_off(l);
+        const __nv_bfloat16 *d = dZ + dz_off(l, rows) + n;
+        float(*sS)[4] = reinterpret_cast<float(*)[4]>(&sH[0][0]);
+        float total = 0.f;
+        for (int b0 = 0; b0 < rows / BLOCK; b0 += GRAD_THREADS) {
+            const int b = b0 + tid;
+            if (b < rows / BLOCK) {
+                float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 16
+                for (int r = 0; r < BLOCK; ++r) {
+                    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(d + (size_t)(b * BLOCK + r) * N));
+                    const float2 p = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v.x));
+                    const float2 q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v.y));
+                    s[0] += p.x;
+                    s[1] += p.y;
+                    s[2] += q.x;
+                    s[3] += q.y;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) sS[tid][k] = s[k];
+            }
+            __syncthreads();
+            if (tid < 4) {
+                const int nb = min(GRAD_THREADS, rows / BLOCK - b0);
+                for (int k = 0; k < nb; ++k) total += sS[k][tid];
+            }
+            __syncthreads();
+        }
+        if (tid < 4) grad_b[c + tid] = total;
+        return;
     }
+    int q = blockIdx.x, l = 0;
+    while (l < NL - 1 && q >= grad_tiles(l)) q -= grad_tiles(l++);
+    const int K = layer_in(l), N = layer_out(l);
+    const int m0 = q / grad_ngroups(l) * GM, n0 = q % grad_ngroups(l) * GN;
+    const int ncol = min(GN, N - n0);   // 32, or 16 in the last group of the output layer
+    const __nv_bfloat16 *h = (l == 0 ? H0 : Hh + (size_t)(l - 1) * nrows * HID) + m0;
+    const __nv_bfloat16 *d = dZ + dz_off(l, rows) + n0;
+    const int chunks = (rows + GCH - 1) / GCH;
+    auto issue = [&](int ch) {
+        const int r0 = ch * GCH, s = ch % GST;
+        if (h16) {
+            for (int k = tid; k < GCH * GM / 8; k += GRAD_THREADS) {
+                const int r = k / (GM / 8), c = 8 * (k % (GM / 8));
+                const bool in = r0 + r < nrows;
+                cp16(&sH[s][r * SHS + c], h + (in ? (size_t)(r0 + r) * K + c : 0), in);
+            }
+        } else {   // layer inputs not on 16-byte boundaries: pairs
+            for (int k = tid; k < GCH * GM / 2; k += GRAD_THREADS) {
+                const int r = k / (GM / 2), c = 2 * (k % (GM / 2));
+                *reinterpret_cast<uint32_t *>(&sH[s][r * SHS + c]) =
+                    r0 + r < nrows ? *reinterpret_cast<const uint32_t *>(h + (size_t)(r0 + r) * K + c) : 0u;
+            }
+        }
+        for (int k = tid; k < GCH * GN / 8; k += GRAD_THREADS) {
+            const int r = k / (GN / 8), c = 8 * (k % (GN / 8));
+            const bool in = r0 + r < rows && c < ncol;
+            cp16(&sD[s][r * SDS + c], d + (in ? (size_t)(r0 + r) * N + c : 0), in);
+        }
+    };
+#pragma unroll
+    for (int ch = 0; ch < GST - 1; ++ch) {
+        if (ch < chunks) issue(ch);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+    const int ra = (lane & 7) + ((lane >> 4) & 1) * 8, ca = ((lane >> 3) & 1) * 8;   // A: H^T, transposed reads
+    const int rb = lane, cb = 8 * wp;                                               // B: dZ, 32 samples
+    for (int ch = 0; ch < chunks; ++ch) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GST - 2) : "memory");
+        __syncthreads();   // chunk ch is in shared memory, chunk ch - 1 consumed
+        if (ch + GST - 1 < chunks) issue(ch + GST - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const int s = ch % GST;
+        // the chunk's blocks are independent chains, then added in their order (blocks past the last
+        // sample are zeros)
+        constexpr int NB = GCH / BLOCK;
+        float acc[NB][4];
+#pragma unroll
+        for (int bk = 0; bk < NB; ++bk) acc[bk][0] = acc[bk][1] = acc[bk][2] = acc[bk][3] = 0.f;
+        const __nv_bfloat16 *ph = &sH[s][ra * SHS + ca], *pd = &sD[s][rb * SDS + cb];
+#pragma unroll
+        for (int k2 = 0; k2 < 2; ++k2) {
+            uint32_t b[NB][4];
+#pragma unroll
+            for (int bk = 0; bk < NB; ++bk) ldsm_x4_t(b[bk], pd + (bk * BLOCK + 32 * k2) * SDS);
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
+                uint32_t a[NB][4];
+#pragma unroll
+                for (int bk = 0; bk < NB; ++bk) ldsm_x4_t(a[bk], ph + (bk * BLOCK + 32 * k2 + 16 * kk) * SHS);
+#pragma unroll
+                for (int bk = 0; bk < NB; ++bk) mma_bf16(acc[bk], a[bk], b[bk][2 * kk], b[bk][2 * kk + 1]);
+            }
+        }
+#pragma unroll
+        for (int bk = 0; bk < NB; ++bk)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) sum[k] += acc[bk][k];
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (8 * wp >= ncol) return;
+    const int g = lane >> 2, t = lane & 3;
+    float *gw = grad_w + w_off(l) + (size_t)(m0 + g) * N + n0 + 8 * wp + 2 * t;
+    *reinterpret_cast<float2 *>(gw) = make_float2(sum[0], sum[1]);
+    *reinterpret_cast<float2 *>(gw + (size_t)8 * N) = make_float2(sum[2], sum[3]);
 }
 
 // Adam on the FP32 master weights [in][out] and biases; refresh both bf16 layouts
@@ -540,6 +628,41 @@ int check(const char *where) {
 
 }  // namespace
 
+// beta^step as the FP32 product of its factors, one after another.  A training loop asks for one step after
+// the other, so a thread goes on from the product of its last call where beta is the same (a whole
+// product per call takes 25 us at step 16000); the value does not depend on it.
+float power(float beta, int step, int slot) {
+    struct Last {
+        float beta = 0.f, prod = 1.f;
+        int step = 0;
+    };
+    static thread_local Last last[2];
+    Last &l = last[slot];
+    const int to = step < 100000 ? step : 100000;
+    if (l.beta != beta || l.step > to) l = Last{beta, 1.f, 0};
+    for (; l.step < to; ++l.step) l.prod *= beta;
+    return l.prod;
+}
+
+// the kernels' shared-memory limits (per device, set once: an attribute of the function)
+int dynamic_smem() {
+    static std::mutex mu;
+    static bool done[64] = {false};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    if (e == cudaSuccess && dev >= 0 && dev < 64 && done[dev]) return VL_OK;
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MLP_SMEM);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(mlp_backprop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MLP_SMEM);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GRAD_SMEM);
+    if (e != cudaSuccess) return fail(VL_ERR_CUDA, cudaGetErrorString(e));
+    if (dev >= 0 && dev < 64) done[dev] = true;
+    return VL_OK;
+}
+
 extern "C" {
 
 VL_API int vl_closure_features(const void *f, int32_t prec, int32_t nx, int32_t nu, int32_t nv,
@@ -605,18 +728,18 @@ VL_API int vl_mlp_forward(const float *X, int32_t nrows, const void *wf, const v
     if (nrows == 0) return VL_OK;
     const bool save = H0 || Hh || Z;
     if (save && !(H0 && Hh && Z)) return fail(VL_ERR_INVALID, "training forward needs H0, Hh and Z");
-    const int tiles = (nrows + 15) / 16;
-    int blocks = (tiles + WARPS - 1) / WARPS;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    mlp_forward_kernel<<<blocks, 32 * WARPS, 0, static_cast<cudaStream_t>(stream)>>>(
+    int rc = dynamic_smem();
+    if (rc) return rc;
+    mlp_forward_kernel<<<(nrows + ROWS - 1) / ROWS, 32 * WARPS, MLP_SMEM, static_cast<cudaStream_t>(stream)>>>(
         X, nrows, weights_of(static_cast<const __nv_bfloat16 *>(wf), static_cast<const __nv_bfloat16 *>(wb), bias),
         Y, static_cast<__nv_bfloat16 *>(H0), static_cast<__nv_bfloat16 *>(Hh), Z);
     return check("mlp_forward_kernel");
 }
 
 VL_API size_t vl_mlp_partial_floats(int32_t nrows) {
-    const size_t blocks = (size_t)(nrows + ROWS - 1) / ROWS;
-    return blocks * (GW_ELEMS + GB_ELEMS);
+    // dZ of every layer, bf16, rows up to a multiple of BLOCK
+    const size_t rows = ((size_t)nrows + BLOCK - 1) / BLOCK * BLOCK;
+    return rows * (3 * HID + OUT) / 2 + 4;   // (+ a 16-byte boundary at its start)
 }
 
 VL_API int vl_mlp_backward(const float *Y, const float *T, int32_t nrows, int32_t nout, const void *wf,
@@ -626,19 +749,19 @@ VL_API int vl_mlp_backward(const float *Y, const float *T, int32_t nrows, int32_
         return fail(VL_ERR_INVALID, "null argument");
     if (nrows < 1 || nout < 1 || nout > OUT) return fail(VL_ERR_INVALID, "nrows >= 1, nout in 1..48");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int blocks = (nrows + ROWS - 1) / ROWS;
-    float *gw_part = partials;
-    float *gb_part = partials + (size_t)blocks * GW_ELEMS;
-    mlp_backward_kernel<<<blocks, 32 * WARPS, 0, s>>>(
-        Y, T, nrows, nout,
-        weights_of(static_cast<const __nv_bfloat16 *>(wf), static_cast<const __nv_bfloat16 *>(wb), bias),
-        static_cast<const __nv_bfloat16 *>(H0), static_cast<const __nv_bfloat16 *>(Hh), Z, gw_part, gb_part);
-    int rc = check("mlp_backward_kernel");
+    const int rows = (nrows + BLOCK - 1) / BLOCK * BLOCK;
+    __nv_bfloat16 *dZ = reinterpret_cast<__nv_bfloat16 *>((reinterpret_cast<uintptr_t>(partials) + 15) & ~(uintptr_t)15);
+    const bool h16 = ((reinterpret_cast<uintptr_t>(H0) | reinterpret_cast<uintptr_t>(Hh)) & 15) == 0;
+    int rc = dynamic_smem();
     if (rc) return rc;
-    mlp_reduce_kernel<<<148 * 4, 256, 0, s>>>(gw_part, blocks, GW_ELEMS, grad_w);
-    if ((rc = check("mlp_reduce_kernel(w)"))) return rc;
-    mlp_reduce_kernel<<<4, 128, 0, s>>>(gb_part, blocks, GB_ELEMS, grad_b);
-    return check("mlp_reduce_kernel(b)");
+    mlp_backprop_kernel<<<rows / ROWS, 32 * WARPS, MLP_SMEM, s>>>(
+        Y, T, nrows, nout,
+        weights_of(static_cast<const __nv_bfloat16 *>(wf), static_cast<const __nv_bfloat16 *>(wb), bias), Z, dZ, rows);
+    if ((rc = check("mlp_backprop_kernel"))) return rc;
+    mlp_grad_kernel<<<GRAD_TILES + BIAS_CTAS, GRAD_THREADS, GRAD_SMEM, s>>>(static_cast<const __nv_bfloat16 *>(H0),
+                                                                    static_cast<const __nv_bfloat16 *>(Hh), dZ, nrows,
+                                                                    rows, h16, grad_w, grad_b);
+    return check("mlp_grad_kernel");
 }
 
 VL_API int vl_mlp_adam(float *master_w, float *master_b, const float *grad_w, const float *grad_b, float *m_w,
@@ -646,13 +769,7 @@ VL_API int vl_mlp_adam(float *master_w, float *master_b, const float *grad_w, co
                        float beta2, float eps, int32_t step, float weight_decay, void *stream) {
     if (!master_w || !master_b || !grad_w || !grad_b || !m_w || !v_w || !m_b || !v_b || !wf || !wb || step < 1)
         return fail(VL_ERR_INVALID, "null argument or step < 1");
-    float bc1 = 1.f, bc2 = 1.f;
-    for (int i = 0; i < step && i < 100000; ++i) {
-        bc1 *= beta1;
-        bc2 *= beta2;
-    }
-    bc1 = 1.f - bc1;
-    bc2 = 1.f - bc2;
+    const float bc1 = 1.f - power(beta1, step, 0), bc2 = 1.f - power(beta2, step, 1);
     mlp_adam_kernel<<<148 * 2, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         master_w, master_b, grad_w, grad_b, m_w, v_w, m_b, v_b, static_cast<__nv_bfloat16 *>(wf),
         static_cast<__nv_bfloat16 *>(wb), lr, beta1, beta2, eps, bc1, bc2, weight_decay);
