@@ -1119,10 +1119,12 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
     //     even); the line form elsewhere (n = 7 at 24x31x33, odd rows: 66 / 90 us per Euler /
     //     combination stage against 119 / 147 in the generic kernel's cp.async form; on 16-byte rows the
     //     TMA form is faster: 83 / 89 against 88 / 121 us at 32^3)
-    //   FP32, other orders: the line form (64^3, n = 9: 703 / 865 us against 870 / 912 in the generic
-    //     kernel's paired-row TMA form; n = 7 at 24x31x33 32 / 40 against 56 / 63 in the register-pencil
-    //     kernel; n = 4 at 32x64x64 27 / 32 against 40 / 48 in the order-4 TMA kernel; n = 6 at 32^3
-    //     26.6 / 30.9 against 27.9 / 30.4 in the generic kernel's TMA form)
+    //   FP32, orders 2 to 6: the generic kernel's TMA forms where the rows allow them (n = 6 at 32x62x62
+    //     91 / 100 us against 97 / 116 in the line form, n = 4 26 / 28 against 27 / 31 and 39 / 46 in the
+    //     order-4 TMA kernel, n = 2 at 64x128x128 31 / 33 against 44 / 49)
+    //   FP32, other orders and rows: the line form (64^3, n = 9: 703 / 865 us against 870 / 912 in the
+    //     generic kernel's paired-row TMA form; n = 7 at 32x62x62 151 / 179 against 179 / 188 in its TMA
+    //     form, at 24x31x33 32 / 40 against 56 / 63 in the register-pencil kernel)
     // The line form takes x slabs below 4 GiB (32-bit offsets); beyond, the generic and register-pencil
     // kernels serve its cases.  VLASOV1D2V_STAGE_KERNEL=frag|gen|pencil|line selects one of the forms
     // that apply, for comparisons; VLASOV1D2V_GEN_NO_TMA=1 keeps the generic kernel off its TMA forms.
@@ -1137,6 +1139,7 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
                             ((size_t)(cfg->nu + 2) * n) % 2 == 0 && !no_gen_tma && encode_fn() != nullptr;
     const bool line_ok = elems / (size_t)(cfg->nx + 2) * (cfg->precision == VL_FP64 ? 8 : 4) < ((size_t)1 << 32);
     const bool tma64 = ((size_t)(cfg->nv + 2) * n) % 2 == 0 && encode_fn() != nullptr && !no_gen_tma;
+    const bool tma_better = cfg->precision == VL_FP64 ? tma64 : (gen_tma32 || gen_pair32) && n >= 2 && n <= 6;
     // the forms without the line kernel (they also say how the entry points want buffers aligned)
     const int general = cfg->precision == VL_FP64     ? VL_STAGE_GEN
                         : c->use_tma                  ? VL_STAGE_TMA
@@ -1146,7 +1149,8 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
                      : cfg->precision == VL_FP64                                       ? 8
                                                                                        : 4;
     c->stage_kernel = c->use_frag                                      ? VL_STAGE_FRAG
-                      : line_ok && !(cfg->precision == VL_FP64 && tma64) ? VL_STAGE_LINE
+                      : tma_better                                     ? VL_STAGE_GEN
+                      : line_ok                                        ? VL_STAGE_LINE
                                                                        : general;
     {
         const char *env = getenv("VLASOV1D2V_STAGE_KERNEL");
