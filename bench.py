@@ -581,8 +581,8 @@ def main():
                    "buffers, 3 buffers)", "parallelism": f"replicas x{world}"},
         "roofline": head["roofline"],
         "e2e": head["e2e"],
-        # per step: 3 fused stage kernels + 3 cluster field solves; one moment per call
-        "gpu_launches": 6 * args.steps + 1,
+        # per step: 3 stage kernels, which solve for the field; one moment and one close per call
+        "gpu_launches": 3 * args.steps + 2,
         "clocks": ck,
         "variants": {"fp32_mixed": {"value": out["fp32"]["value"], "dtype": "f32",
                                     "ms_per_step": out["fp32"]["ms_per_step"],

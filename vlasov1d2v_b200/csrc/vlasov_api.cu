@@ -25,6 +25,7 @@
 #include "vlasov_stage_f32.cuh"
 #include "vlasov_field.cuh"
 #include "vlasov_field_conv.cuh"
+#include "vlasov_field_fuse.cuh"
 #include "vlasov_stage_gen.cuh"
 #include "vlasov_gen_kinds.h"
 #include "vlasov_line.h"
@@ -703,6 +704,30 @@ int stage_occupancy(int n, bool tma, bool frag, bool gen, bool gtma, bool gpair)
     }
 }
 
+// one pipeline stage of the generic kernel's TMA forms, 0 where they have no form with the field solve
+template <int N, typename T>
+size_t gen_fuse_room_t(bool pair) {
+    if (!vl::gen_fusable<T>(N, pair)) return 0;
+    return pair ? vl::GenPairGeom<N, T>::STAGE_B : vl::GenTmaGeom<N, T>::STAGE_B;
+}
+
+template <typename T>
+size_t gen_fuse_room(int n, bool pair) {
+    switch (n) {
+        case 1: return gen_fuse_room_t<1, T>(pair);
+        case 2: return gen_fuse_room_t<2, T>(pair);
+        case 3: return gen_fuse_room_t<3, T>(pair);
+        case 4: return gen_fuse_room_t<4, T>(pair);
+        case 5: return gen_fuse_room_t<5, T>(pair);
+        case 6: return gen_fuse_room_t<6, T>(pair);
+        case 7: return gen_fuse_room_t<7, T>(pair);
+        case 8: return gen_fuse_room_t<8, T>(pair);
+        case 9: return gen_fuse_room_t<9, T>(pair);
+        case 10: return gen_fuse_room_t<10, T>(pair);
+        default: return 0;
+    }
+}
+
 // v elements per stage tile of the generic kernel
 template <typename T>
 int gen_ept(int n) {
@@ -908,6 +933,9 @@ size_t partials_bytes(const vl_ctx *c) {
     return (b + 255) & ~(size_t)255;
 }
 
+// a control record of the loop whose stage kernels solve for the field
+constexpr size_t CONTROL_BYTES = (sizeof(vl_run_state) + 255) & ~(size_t)255;
+
 vl::ScalarArgs scalar_args(const vl_ctx *c, const double *E) {
     vl::ScalarArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -954,6 +982,81 @@ int upload(P **dst, const void *src, size_t bytes) {
     VL_CUDA(cudaMalloc((void **)dst, bytes));
     VL_CUDA(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
     return VL_OK;
+}
+
+// The loop with the field solves inside the stage kernels: three launches a step, and one at the end
+// that closes the last step.
+int fused_steps(vl_ctx *c, void *f, void *sa, void *sb, double *E, double *phi, vl_run_state *state, void *workspace,
+                int nsteps, cudaStream_t s) {
+    char *w = static_cast<char *>(workspace);
+    double *parts[2] = {reinterpret_cast<double *>(w), reinterpret_cast<double *>(w + partials_bytes(c))};
+    vl_run_state *ctl[2];
+    for (int k = 0; k < 2; ++k)
+        ctl[k] = reinterpret_cast<vl_run_state *>(w + 2 * partials_bytes(c) + k * CONTROL_BYTES);
+    int rc, cur = 0;
+    if ((rc = moment(c, f, parts[0], c->moment_grid_g, s))) return rc;
+    vl::StageArgs st = stage_args(c);
+    st.err = &state->status;
+    st.xhalo = VL_XHALO_PERIODIC;
+    vl::FieldFuse &ff = st.ff;
+    ff.KE = c->d_ke;
+    ff.KP = c->d_kp;
+    ff.kappa = c->cfg.kappa;
+    ff.status = &state->status;
+    ff.st = state;
+    ff.E_prev = E;
+    ff.xw = c->d_xw;
+    ff.dx = c->cfg.dx;
+    ff.du = c->cfg.du;
+    ff.dv = c->cfg.dv;
+    ff.umax = c->cfg.umax;
+    ff.vmax = c->cfg.vmax;
+    ff.courant = c->cfg.courant;
+    ff.G = c->moment_grid_g;
+    auto go = [&](const void *in, const void *fn, void *out) {
+        st.in = in;
+        st.fn = fn;
+        st.out = out;
+        ff.partials = parts[cur];
+        st.partials = parts[cur ^ 1];
+        cur ^= 1;
+        const int r = stage(c, st, s);
+        ff.G = (int)stage_grid(c, st).x;   // of the partials just written
+        return r;
+    };
+    for (int it = 0; it < nsteps; ++it) {
+        // stage 0: E(f^n); s0 = f + dt R(f); the step before closed first
+        ff.mode = it == 0 ? vl::FUSE_FIRST : vl::FUSE_STEP;
+        ff.ctl_in = it == 0 ? state : ctl[it & 1];
+        ff.ctl_out = ctl[(it + 1) & 1];
+        ff.E_out = ff.phi_out = nullptr;
+        st.state = nullptr;
+        st.dt = nullptr;
+        st.kind = vl::KIND_EULER;
+        st.ghost_out = f;
+        if ((rc = go(f, nullptr, sa))) return rc;
+        // stage 1: E(s0); s1 = 3/4 f + 1/4 s0 + 1/4 dt R(s0)
+        ff.mode = vl::FUSE_FIELD;
+        st.state = ff.ctl_out;
+        st.dt = &ff.ctl_out->dt;
+        st.kind = vl::KIND_COMBINE;
+        st.ghost_out = nullptr;
+        st.c0 = kRK3[0][0];
+        st.c1 = kRK3[0][1];
+        st.c2 = kRK3[0][2];
+        if ((rc = go(sa, f, sb))) return rc;
+        // stage 2: E(s1), the field the caller gets; f <- 1/3 f + 2/3 s1 + 2/3 dt R(s1)
+        ff.E_out = E;
+        ff.phi_out = phi;
+        st.c0 = kRK3[1][0];
+        st.c1 = kRK3[1][1];
+        st.c2 = kRK3[1][2];
+        if ((rc = go(sb, f, f))) return rc;
+    }
+    if (nsteps == 0) return VL_OK;
+    ff.ctl_in = ctl[nsteps & 1];
+    vl::field_close_kernel<<<1, 256, 0, s>>>(ff, c->cfg.nx, c->cfg.n, c->cfg.accel, c->cfg.bfield);
+    return check_launch("field_close_kernel");
 }
 
 }  // namespace
@@ -1177,6 +1280,8 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
     c->stage_grid_g = grid_for(occ);
     c->stage_slots = c->sm_count * occ;
     c->stage_tiles = tiles;
+    int slots1 = c->stage_slots;   // of the Euler stage's kernel
+    if (c->use_frag && cfg->precision == VL_FP64) slots1 = c->sm_count * frag_nofn_occupancy();
     c->stage_grid_g1 = (c->use_frag && cfg->precision == VL_FP64) ? grid_for(frag_nofn_occupancy())
                                                                   : c->stage_grid_g;
     if (c->stage_kernel == VL_STAGE_LINE) {
@@ -1188,7 +1293,28 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
         c->stage_grid_g = line_grid(lo);
         c->stage_slots = c->sm_count * lo;
         c->stage_tiles = lt;
-        c->stage_grid_g1 = line_grid(std::min(occ_of(vl::KIND_EULER), occ_of(vl::KIND_RHS)));
+        const int lo1 = std::min(occ_of(vl::KIND_EULER), occ_of(vl::KIND_RHS));
+        c->stage_grid_g1 = line_grid(lo1);
+        slots1 = c->sm_count * lo1;
+    }
+    {
+        // the field solve inside the stage kernels: tables, a kernel that has the prologue, room for the
+        // nx n densities (VLASOV1D2V_FIELD=solve keeps separate solves, for comparisons)
+        const size_t room = c->use_frag ? (cfg->precision == VL_FP64 ? vl::FragGeom<double, false>::STAGE_B
+                                                                     : vl::FragGeom<float>::STAGE_B)
+                            : c->stage_kernel == VL_STAGE_LINE
+                                ? (cfg->precision == VL_FP64 ? vl::line_smem<double>(n) : vl::line_smem<float>(n))
+                            : !(c->gen_tma || c->gen_pair) ? 0
+                            : cfg->precision == VL_FP64    ? gen_fuse_room<double>(n, false)
+                                                           : gen_fuse_room<float>(n, c->gen_pair);
+        const char *env = getenv("VLASOV1D2V_FIELD");
+        // (a CTA that starts in a later wave repeats the solve where the SMs would have stages to run: on
+        // grids of more than one wave separate solves are as fast or faster, n = 8 at 64x32x32 501 against
+        // 509 us per step; in one wave the fused form is, 57 against 67 us at 16x20x20 n = 6, 579 against
+        // 594 at 32x50x50 n = 8)
+        const bool one_wave = c->stage_grid_g * cfg->nx <= c->stage_slots && c->stage_grid_g1 * cfg->nx <= slots1;
+        c->fuse_field = c->d_ke != nullptr && one_wave && room >= vl::field_fuse_scratch(cfg->nx, n) &&
+                        !(env && std::string(env) == "solve");
     }
     // standalone moment: MOMENT_CTAS_PER_SM resident CTAs per SM, at most one per u element
     int gm = (c->sm_count * vl::MOMENT_CTAS_PER_SM) / cfg->nx;
@@ -1232,7 +1358,8 @@ size_t vl_state_elems(const vl_ctx *c) {
 
 size_t vl_workspace_bytes(const vl_ctx *c) {
     if (c == nullptr) return 0;
-    return partials_bytes(c);
+    // (stage kernels that solve for the field read and write different partials, and control records)
+    return c->fuse_field ? 2 * partials_bytes(c) + 2 * CONTROL_BYTES : partials_bytes(c);
 }
 
 int vl_rhs(vl_ctx *c, const void *f, const double *E, void *out, int xhalo, void *stream) {
@@ -1386,6 +1513,7 @@ int vl_ssp_rk3_steps(vl_ctx *c, void *f, void *sa, void *sb, double *E, double *
         return fail(VL_ERR_INVALID, "null argument");
     if (nsteps < 0) return fail(VL_ERR_INVALID, "nsteps < 0");
     cudaStream_t s = as_stream(stream);
+    if (c->fuse_field) return fused_steps(c, f, sa, sb, E, phi, state, workspace, nsteps, s);
     double *partials = static_cast<double *>(workspace);
     const int G = c->stage_grid_g;
     int rc;

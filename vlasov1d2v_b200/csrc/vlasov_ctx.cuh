@@ -45,6 +45,7 @@ struct vl_ctx {
     bool use_tma = false;         // stage kernel: TMA-pipelined form (aligned orders)
     bool use_frag = false;        // n = 8: quad-fragment stage kernel (tensor cores in FP64)
     int stage_kernel = VL_STAGE_GEN;   // which stage kernel the launches use (vl_stage_kernel)
+    bool fuse_field = false;      // the loop's stage kernels solve for E themselves (vlasov_field_fuse.cuh)
     int state_align = 4;          // alignment that the entry points ask of state buffers (bytes)
     bool gen_tma = false;         // generic stage kernel in its TMA form (FP64, aligned rows)
     bool gen_pair = false;        // generic stage kernel in its paired-row TMA form (FP32, R = 2 mod 4)

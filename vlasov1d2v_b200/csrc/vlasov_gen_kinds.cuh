@@ -9,15 +9,15 @@
 namespace vl {
 namespace gk {
 
-template <typename T, int N, bool PAIR, int K, int B>
+template <typename T, int N, bool PAIR, int K, int B, bool FUSE = false>
 constexpr auto kernel() {
     if constexpr (PAIR)
-        return &stage_gen_pair_kernel<N, T, K, B>;
+        return &stage_gen_pair_kernel<N, T, K, B, FUSE>;
     else
-        return &stage_gen_tma_kernel<N, T, K, B>;
+        return &stage_gen_tma_kernel<N, T, K, B, FUSE>;
 }
 
-template <typename T, int N, bool PAIR, int K, int B>
+template <typename T, int N, bool PAIR, int K, int B, bool FUSE = false>
 cudaError_t launch_one(dim3 grid, size_t smem, cudaStream_t s, const StageArgs &a, const StageTables<T> &tb,
                        const GenMaps &maps) {
     constexpr int THREADS = PAIR ? GenPairGeom<N, T>::THREADS : GenTmaGeom<N, T>::THREADS;
@@ -27,13 +27,24 @@ cudaError_t launch_one(dim3 grid, size_t smem, cudaStream_t s, const StageArgs &
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    return cudaLaunchKernelEx(&cfg, kernel<T, N, PAIR, K, B>(), a, tb, maps);
+    return cudaLaunchKernelEx(&cfg, kernel<T, N, PAIR, K, B, FUSE>(), a, tb, maps);
 }
 
 template <typename T, int N, bool PAIR>
 cudaError_t launch_n(int kind, bool bg, dim3 grid, size_t smem, cudaStream_t s, const StageArgs &a,
                      const StageTables<T> &tb, const GenMaps &maps) {
     constexpr bool HAS_BG = sizeof(T) == 4;   // the background split is a form of FP32 states
+    if constexpr (gen_fusable<T>(N, PAIR)) {
+        if (a.ff.mode != FUSE_NONE) {
+            if (HAS_BG && bg) {
+                constexpr int B1 = HAS_BG ? 1 : 0;
+                if (kind == KIND_EULER) return launch_one<T, N, PAIR, KIND_EULER, B1, true>(grid, smem, s, a, tb, maps);
+                return launch_one<T, N, PAIR, KIND_COMBINE, B1, true>(grid, smem, s, a, tb, maps);
+            }
+            if (kind == KIND_EULER) return launch_one<T, N, PAIR, KIND_EULER, 0, true>(grid, smem, s, a, tb, maps);
+            return launch_one<T, N, PAIR, KIND_COMBINE, 0, true>(grid, smem, s, a, tb, maps);
+        }
+    }
     if (kind == KIND_EULER) {
         if (HAS_BG && bg) return launch_one<T, N, PAIR, KIND_EULER, HAS_BG ? 1 : 0>(grid, smem, s, a, tb, maps);
         return launch_one<T, N, PAIR, KIND_EULER, 0>(grid, smem, s, a, tb, maps);
@@ -52,6 +63,13 @@ void prepare_n(size_t smem) {
     cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_EULER, 0>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
     cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_COMBINE, 0>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
     cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_RHS, 0>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if constexpr (gen_fusable<T>(N, PAIR)) {
+        constexpr int B1 = sizeof(T) == 4 ? 1 : 0;
+        cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_EULER, 0, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+        cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_COMBINE, 0, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+        cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_EULER, B1, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+        cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_COMBINE, B1, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    }
     if constexpr (sizeof(T) == 4) {
         cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_EULER, 1>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
         cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_COMBINE, 1>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);

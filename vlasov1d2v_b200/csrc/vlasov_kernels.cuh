@@ -42,6 +42,29 @@ struct StageTables {
     double wv[NMAX];
 };
 
+// Field solve and loop bookkeeping inside a stage kernel (vlasov_field_fuse.cuh)
+enum FuseMode : int {
+    FUSE_NONE = 0,    // E is given
+    FUSE_FIELD = 1,   // E from the moment partials of the stage's input
+    FUSE_FIRST = 2,   // the same, first stage of a batch's first step: promotes the loop state
+    FUSE_STEP = 3,    // the same, first stage of a later step: closes the step before it first
+};
+struct FieldFuse {
+    int mode;
+    int G;                       // partials per x node
+    const double *partials;      // [nx][G][n] of the stage's input (not the buffer the stage writes)
+    const double *KE, *KP;       // convolution tables
+    double kappa;
+    double *E_out, *phi_out;     // written by the CTAs with blockIdx.x = 0, or null
+    int *status;                 // bit 0: non-finite E
+    const vl_run_state *ctl_in;  // control record of the step before (FUSE_FIRST: the loop state)
+    vl_run_state *ctl_out;       // control record of this step
+    vl_run_state *st;            // the loop state: limits, history ring, status
+    const double *E_prev;        // the field of the step before (its last solve)
+    const double *xw;
+    double dx, du, dv, umax, vmax, courant;
+};
+
 struct StageArgs {
     const void *in;        // stage input (ghost-inclusive)
     const void *fn;        // f^n for KIND_COMBINE
@@ -72,6 +95,7 @@ struct StageArgs {
     // context's Jacobians; a call with other direction weights (jx, jv above) scales them by
     // jx / J_x and jv / J_v (the RHS kind only; the RK stages use the context's Jacobians)
     double sx, sv;
+    FieldFuse ff;
     int grid_g;  // CTAs per x element (0: the context's own choice; host side)
     int never;   // line-form kernel: a value that no tile index takes (-1)
 };

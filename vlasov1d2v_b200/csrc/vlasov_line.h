@@ -23,11 +23,18 @@ template <typename T>
 int line_occupancy(int n, int kind);
 // v elements per tile
 int line_ept(int n);
+// dynamic shared memory of a CTA (bytes)
+template <typename T>
+size_t line_smem(int n);
 
 template <>
 cudaError_t line_launch<double>(int n, const StageArgs &a, const LineCoef &lc, dim3 grid, cudaStream_t s);
 template <>
 cudaError_t line_launch<float>(int n, const StageArgs &a, const LineCoef &lc, dim3 grid, cudaStream_t s);
+template <>
+size_t line_smem<double>(int n);
+template <>
+size_t line_smem<float>(int n);
 template <>
 int line_occupancy<double>(int n, int kind);
 template <>

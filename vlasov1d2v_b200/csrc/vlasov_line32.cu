@@ -10,6 +10,11 @@ cudaError_t line_launch<float>(int n, const StageArgs &a, const LineCoef &lc, di
 }
 
 template <>
+size_t line_smem<float>(int n) {
+    return lk::with_order(n, (size_t)0, [](auto nc) { return LineGeom<decltype(nc)::value, float>::smem_bytes(); });
+}
+
+template <>
 int line_occupancy<float>(int n, int kind) {
     return lk::with_order(n, 1, [&](auto nc) { return lk::occupancy<decltype(nc)::value, float>(kind); });
 }

@@ -10,6 +10,11 @@ cudaError_t line_launch<double>(int n, const StageArgs &a, const LineCoef &lc, d
 }
 
 template <>
+size_t line_smem<double>(int n) {
+    return lk::with_order(n, (size_t)0, [](auto nc) { return LineGeom<decltype(nc)::value, double>::smem_bytes(); });
+}
+
+template <>
 int line_occupancy<double>(int n, int kind) {
     return lk::with_order(n, 1, [&](auto nc) { return lk::occupancy<decltype(nc)::value, double>(kind); });
 }

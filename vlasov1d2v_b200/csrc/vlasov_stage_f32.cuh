@@ -28,6 +28,7 @@
 
 #include <type_traits>
 
+#include "vlasov_field_fuse.cuh"
 #include "vlasov_kernels.cuh"
 #include "vlasov_stage_frag.cuh"
 #include "vlasov_stage_tma.cuh"
@@ -70,6 +71,7 @@ stage_f32_kernel(const StageArgs a, const __grid_constant__ F32Tables tb, const 
         (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
     __shared__ __align__(8) uint64_t full[2];
     __shared__ dd sRed[N];
+    __shared__ FuseShared<N, G::THREADS> sFuse;
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -141,16 +143,27 @@ stage_f32_kernel(const StageArgs a, const __grid_constant__ F32Tables tb, const 
     };
     if (tid == 0) {
         if (ntile_cta > 0) issue(0, 0);
-        if (ntile_cta > 1) issue(1, 1);
+        if (a.ff.mode == FUSE_NONE && ntile_cta > 1) issue(1, 1);
+    }
+    if (KIND != KIND_RHS && a.ff.mode != FUSE_NONE) {
+        // E at this x element while the first tile travels; the second stage is the scratch
+        if (!field_prologue<N, G::THREADS>(a, e, reinterpret_cast<double *>(stage_ptr(1)), sFuse)) {
+            if (ntile_cta > 0) mbar_wait_bounded(&full[0], 0);   // no copy left in flight
+            return;
+        }
+        if (tid == 0 && ntile_cta > 1) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            issue(1, 1);
+        }
     }
 
     const double accel = a.accel, bfield = a.bfield;
-    const double dtd = (KIND == KIND_RHS) ? 0.0 : *a.dt;
+    const double dtd = (KIND == KIND_RHS) ? 0.0 : a.ff.mode != FUSE_NONE ? sFuse.dt : *a.dt;
     const float2 dt2 = f2s((float)dtd), c12 = f2s((float)a.c1), c2dt2 = f2s((float)(a.c2 * dtd));
     const float2 mone = f2s(-1.0f);
     const float ju = (float)a.ju;
     const float rsx = (float)a.sx, rsv = (float)a.sv;
-    const double Ei = a.E[Eg * N + g];
+    const double Ei = a.ff.mode != FUSE_NONE ? sFuse.E[g] : a.E[Eg * N + g];
     const float2 Ei2 = f2s((float)Ei);
     // per-thread coefficients: x rows g (pairs), v rows k0, k1 (pairs over m), both upwind variants
     // of the folded columns, and the neighbour-trace coefficients

@@ -35,6 +35,7 @@
 
 #include <type_traits>
 
+#include "vlasov_field_fuse.cuh"
 #include "vlasov_kernels.cuh"
 #include "vlasov_stage.cuh"
 #include "vlasov_stage_tma.cuh"
@@ -135,6 +136,7 @@ stage_frag_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
         (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
     __shared__ __align__(8) uint64_t full[2];
     __shared__ dd sRed[EPT * G::JS][N];
+    __shared__ FuseShared<N, NT> sFuse;
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -202,14 +204,25 @@ stage_frag_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
     };
     if (tid == 0) {
         if (ntile_cta > 0) issue(0, 0);
-        if (ntile_cta > 1) issue(1, 1);
+        if (a.ff.mode == FUSE_NONE && ntile_cta > 1) issue(1, 1);
+    }
+    if (KT != KIND_RHS && a.ff.mode != FUSE_NONE) {
+        // E at this x element while the first tile travels; the second stage is the scratch
+        if (!field_prologue<N, NT>(a, e, reinterpret_cast<double *>(stage_ptr(1)), sFuse)) {
+            if (ntile_cta > 0) mbar_wait_bounded(&full[0], 0);   // no copy left in flight
+            return;
+        }
+        if (tid == 0 && ntile_cta > 1) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            issue(1, 1);
+        }
     }
 
     const double accel = a.accel, bfield = a.bfield;
-    const double dtd = (kind == KIND_RHS) ? 0.0 : *a.dt;
+    const double dtd = (kind == KIND_RHS) ? 0.0 : a.ff.mode != FUSE_NONE ? sFuse.dt : *a.dt;
     const T dtT = (T)dtd, c0 = (T)a.c0, c1 = (T)a.c1, c2dt = (T)(a.c2 * dtd);
     const T jx = (T)a.jx, ju = (T)a.ju, jv = (T)a.jv;
-    const double Ei = a.E[Eg * N + g];
+    const double Ei = a.ff.mode != FUSE_NONE ? sFuse.E[g] : a.E[Eg * N + g];
     // per-thread coefficients (runtime rows g and 2t, 2t + 1 of the tables)
     // MMA form: fragments up[g][t], up[g][4 + t] and their upwind-folded variants (speed >= 0
     // folds the own right trace into column n-1, speed < 0 the own left trace into column 0), so

@@ -46,6 +46,7 @@
 
 #include <type_traits>
 
+#include "vlasov_field_fuse.cuh"
 #include "vlasov_kernels.cuh"
 #include "vlasov_stage_tma.cuh"
 
@@ -292,6 +293,13 @@ struct GenLayout<2, N, T, EPT> {
     static constexpr size_t S_BG = GP::BG_B, S_STAGE = GP::STAGE_B;
 };
 
+// TMA forms with an instantiation that solves for E itself: those the dispatch chooses in FP64 and FP32,
+// but FP32 n = 2 (24x30x30: 45 us per step with separate solves, 52 without)
+template <typename T>
+__host__ __device__ constexpr bool gen_fusable(int n, bool pair) {
+    return sizeof(T) == 8 ? !pair : n >= 3 && n <= 6;
+}
+
 template <typename T>
 struct GenPair;
 template <>
@@ -307,7 +315,8 @@ struct GenPair<float> {
 // partial [e][g][i] (of G per x element).  tb supplies up / xi / wu (compile-time j indices);
 // wfin[k] is the per-column factor of the moment partial (w_k / J_v for the single-problem
 // tables).  smem: GenGeom::smem_bytes() of dynamic shared memory, 128-byte aligned.
-template <int N, typename T, int EPT, typename TB, bool TMA = false, bool PAIR = false, int KT = -1, int BT = -1>
+template <int N, typename T, int EPT, typename TB, bool TMA = false, bool PAIR = false, int KT = -1, int BT = -1,
+          bool FUSE = false>
 __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb, const double *wfin, int e,
                                                int g, int G, unsigned char *smem,
                                                const GenMaps *maps = nullptr) {
@@ -329,6 +338,7 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
     constexpr size_t S_BG = L::S_BG, S_STAGE = L::S_STAGE;
     constexpr int FS = L::FS;        // second face side (elements)
     __shared__ __align__(8) uint64_t gfull[2];   // TMA form: one mbarrier per stage
+    __shared__ FuseShared<FUSE ? N : 1, FUSE ? NT : 32> sFuse;   // field solve in the prologue
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -520,12 +530,39 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
         }
     };
 
+    if constexpr (MB) {
+        if (tid == 0) {
+            if (ntile > 0) issue_tma(0, g);
+            if (!FUSE && ntile > 1) issue_tma(1, g + G);
+        }
+        if constexpr (FUSE) {
+            // E at this x element while the first tile travels; the second stage is the scratch, cleared
+            // again for its pad columns
+            unsigned char *sc = stage_ptr(1);
+            if (!field_prologue<N, NT>(a, e, reinterpret_cast<double *>(sc), sFuse)) {
+                if (ntile > 0) mbar_wait_bounded(&gfull[0], 0);   // no copy left in flight
+                return;
+            }
+            const int nz = (int)((field_fuse_scratch(a.nx, N) + 15) / 16);
+            for (int q = tid; q < nz; q += NT) reinterpret_cast<uint4 *>(sc)[q] = make_uint4(0u, 0u, 0u, 0u);
+            __syncthreads();
+            if (tid == 0 && ntile > 1) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                issue_tma(1, g + G);
+            }
+        }
+    }
+
     const double accel = a.accel, bfield = a.bfield, nbfield = -a.bfield;
     const float kvf = (float)(accel * nbfield);   // FP32 v speed per unit u
-    const double dtd = (kind == KIND_RHS) ? 0.0 : *a.dt;
+    const double dtd = (kind == KIND_RHS) ? 0.0 : FUSE ? sFuse.dt : *a.dt;
     const T dtT = (T)dtd, c0 = (T)a.c0, c1 = (T)a.c1, c2dt = (T)(a.c2 * dtd);
     const T jx = (T)a.jx, ju = (T)a.ju, jv = (T)a.jv;
-    const double Ei = a.E[Eg * N + i];
+    double Ei;
+    if constexpr (FUSE)
+        Ei = sFuse.E[i];
+    else
+        Ei = a.E[Eg * N + i];
     T upi[N], upk0[N], upk1[N];
 #pragma unroll
     for (int m = 0; m < N; ++m) {
@@ -539,12 +576,7 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
     const double wf0 = wfin[k0], wf1 = pad1 ? 0.0 : wfin[k1];
     double mk0 = 0.0, mk1 = 0.0;   // sum_j wu_j out[.., j, k] for the two columns
 
-    if constexpr (TMA) {
-        if (tid == 0) {
-            if (ntile > 0) issue_tma(0, g);
-            if (ntile > 1) issue_tma(1, g + G);
-        }
-    } else {
+    if constexpr (!TMA) {
 #pragma unroll
         for (int s0 = 0; s0 < NST - 1; ++s0) {
             if (s0 < ntile) issue(s0, g + s0 * G);
@@ -829,8 +861,9 @@ stage_gen_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb) {
 
 // TMA form (16-byte-aligned state rows).  KT / BT >= 0 fix the stage kind and the background
 // split at compile time (the instantiations launched by the loop: no per-row branches on them);
-// -1 reads them from the arguments.
-template <int N, typename T, int KT = -1, int BT = -1>
+// -1 reads them from the arguments.  FUSE: the form that solves for E itself (vlasov_field_fuse.cuh), its
+// own instantiation: in one kernel with the other its code costs the n = 9 form registers (64^3: 8%).
+template <int N, typename T, int KT = -1, int BT = -1, bool FUSE = false>
 __global__ void __launch_bounds__(GenTmaGeom<N, T>::THREADS, GenTmaGeom<N, T>::MINB)
 stage_gen_tma_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
                      const __grid_constant__ GenMaps maps) {
@@ -838,12 +871,12 @@ stage_gen_tma_kernel(const StageArgs a, const __grid_constant__ StageTables<T> t
     extern __shared__ __align__(16) unsigned char gen_smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(gen_smem_raw) + 127) & ~(uintptr_t)127);
-    gen_stage_body<N, T, GenGeom<N, T>::EPT, StageTables<T>, true, false, KT, BT>(
+    gen_stage_body<N, T, GenGeom<N, T>::EPT, StageTables<T>, true, false, KT, BT, FUSE>(
         a, tb, tb.wv, blockIdx.y, blockIdx.x, gridDim.x, base, &maps);
 }
 
-// paired-row TMA form (FP32 rows of R = 2 mod 4 floats); KT / BT as for the TMA form
-template <int N, typename T, int KT = -1, int BT = -1>
+// paired-row TMA form (FP32 rows of R = 2 mod 4 floats); KT / BT / FUSE as for the TMA form
+template <int N, typename T, int KT = -1, int BT = -1, bool FUSE = false>
 __global__ void __launch_bounds__(GenPairGeom<N, T>::THREADS, GenPairGeom<N, T>::MINB)
 stage_gen_pair_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
                       const __grid_constant__ GenMaps maps) {
@@ -851,7 +884,7 @@ stage_gen_pair_kernel(const StageArgs a, const __grid_constant__ StageTables<T> 
     extern __shared__ __align__(16) unsigned char gen_smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(gen_smem_raw) + 127) & ~(uintptr_t)127);
-    gen_stage_body<N, T, GenGeom<N, T>::EPT, StageTables<T>, true, true, KT, BT>(
+    gen_stage_body<N, T, GenGeom<N, T>::EPT, StageTables<T>, true, true, KT, BT, FUSE>(
         a, tb, tb.wv, blockIdx.y, blockIdx.x, gridDim.x, base, &maps);
 }
 

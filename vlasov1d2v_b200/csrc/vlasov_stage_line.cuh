@@ -34,6 +34,7 @@
 
 #include <cuda_runtime.h>
 
+#include "vlasov_field_fuse.cuh"
 #include "vlasov_kernels.cuh"
 
 namespace vl {
@@ -204,6 +205,7 @@ stage_line_kernel(const StageArgs a, const __grid_constant__ LineTables<N, T> tb
     T *const sHalo = sTile + 5 * TB;                     // upwind v trace of every row, two buffers
     constexpr int HB = (int)(G::HALO_B / sizeof(T));
     __shared__ float sE[N];
+    __shared__ FuseShared<N, G::THREADS> sFuse;
 
     const int tid = threadIdx.x;
     const int nx = a.nx, nu = a.nu, nv = a.nv;
@@ -242,18 +244,9 @@ stage_line_kernel(const StageArgs a, const __grid_constant__ LineTables<N, T> tb
         b[s] = has ? l / NN : 1 << 20;
         own[s] = (uint32_t)q[s] * sI + (uint32_t)(c[s] & 0xfffff) * ES;
         xrow[s] = (uint32_t)q[s] * sJ + (uint32_t)(c[s] & 0xfffff) * ES;
-        Ei[s] = a.E[Eg * N + q[s]];
     }
     const int hj = tid % N;                                                    // v trace of row tid
     const uint32_t hrow = (uint32_t)(tid / N % N) * sI + (uint32_t)hj * sJ;
-
-    const double accel = a.accel, bfield = a.bfield;
-    const double dtd = (KIND == KIND_RHS) ? 0.0 : *a.dt;
-    const T dtT = (T)dtd, c0 = (T)a.c0, c1 = (T)a.c1, c2dt = (T)(a.c2 * dtd);
-    const T jx = (T)a.jx, ju = (T)a.ju, jv = (T)a.jv;
-    if constexpr (BG == 1) {
-        if (tid < N) sE[tid] = (float)a.E[Eg * N + tid];   // (read after the first barrier)
-    }
 
     const int nbt = (nv + EPT - 1) / EPT;
     const int GX = gridDim.x;
@@ -294,10 +287,22 @@ stage_line_kernel(const StageArgs a, const __grid_constant__ LineTables<N, T> tb
     for (int s = 0; s < L; ++s) mk[s] = 0.0;
 
     int cur = 0;
-    if (au < nu) {
-        load_tile(au, bt);
-        store_tile(0, tile_cols(bt));
+    if (au < nu) load_tile(au, bt);
+    if (KIND != KIND_RHS && a.ff.mode != FUSE_NONE) {
+        // E at this x element while the first tile travels; the tile buffers are the scratch
+        if (!field_prologue<N, G::THREADS>(a, e, reinterpret_cast<double *>(line_smem), sFuse)) return;
     }
+    const double accel = a.accel, bfield = a.bfield;
+    const double dtd = (KIND == KIND_RHS) ? 0.0 : a.ff.mode != FUSE_NONE ? sFuse.dt : *a.dt;
+    const T dtT = (T)dtd, c0 = (T)a.c0, c1 = (T)a.c1, c2dt = (T)(a.c2 * dtd);
+    const T jx = (T)a.jx, ju = (T)a.ju, jv = (T)a.jv;
+    if constexpr (BG == 1) {
+        if (tid < N) sE[tid] = (float)(a.ff.mode != FUSE_NONE ? sFuse.E[tid] : a.E[Eg * N + tid]);   // (read after the first barrier)
+    }
+#pragma unroll
+    for (int s = 0; s < L; ++s) Ei[s] = a.ff.mode != FUSE_NONE ? sFuse.E[q[s]] : a.E[Eg * N + q[s]];
+    if (au < nu) store_tile(0, tile_cols(bt));
+
     while (au < nu) {
         const int ncol = tile_cols(bt), nb = ncol / N;
         const uint32_t toff = tile_off(au, bt);
