@@ -173,6 +173,9 @@ VL_API int vl_run_state_init(vl_ctx *ctx, vl_run_state *state, const double *E0,
                       int64_t max_steps, double *energy_hist, double *time_hist,
                       double *dt_hist, int32_t hist_capacity, double *energy0, void *stream);
 
+/* Copy a host loop state to the device, stream-ordered and without waiting (*host is free on return). */
+VL_API int vl_run_state_write(vl_run_state *state, const vl_run_state *host, void *stream);
+
 /* Stepper.nonlinear_ssp_rk x nsteps (main/timestep.py:141-187) with the main loop's
  * bookkeeping (ts:91-103), entirely on the device: each step runs only while
  * state->time < final_time and steps < max_steps (checked on the device, so extra steps
@@ -303,6 +306,12 @@ VL_API int vl_ens_schedule(vl_ens *ens, int32_t threads, int32_t ctas_per_sm, in
 VL_API int vl_ens_schedule_by_order(vl_ens *ens, int32_t items_per_cta, uint32_t native_orders);
 VL_API int vl_ens_commit(vl_ens *ens);
 VL_API int vl_ens_steps(vl_ens *ens, int32_t nsteps, void *stream);
+/* Around a batch (stream-ordered): vl_ens_begin makes every member that has neither failed nor reached
+ * its final time ready for up to max_steps further steps, its step count from 0; vl_ens_collect gathers
+ * per member, in rows of 2 + 3 k doubles, the steps taken, the status and the first k entries (as far as
+ * taken and kept) of the energy, time and dt histories.                                       */
+VL_API int vl_ens_begin(vl_ens *ens, int64_t max_steps, void *stream);
+VL_API int vl_ens_collect(vl_ens *ens, int32_t k, double *out, void *stream);
 
 /* ---- learned coarse-grid closure ------------------------------------------------------------------
  * No counterpart in the reference.  A per-(x node, velocity element) MLP corrects the RHS of a

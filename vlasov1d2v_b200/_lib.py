@@ -27,7 +27,8 @@ EXPORTED = (
     "vl_sync_stage_ghosts", "vl_rhs_whole",
     "vl_ssp_rk3_steps_noalloc", "vl_initial_state", "vl_smooth_edges", "vl_interpolate",
     "vl_set_background", "vl_set_background_pairs", "vl_ens_create", "vl_ens_destroy", "vl_ens_workspace_bytes", "vl_ens_bind",
-    "vl_ens_schedule", "vl_ens_schedule_by_order", "vl_ens_commit", "vl_ens_steps", "vl_mlp_dims", "vl_mlp_forward",
+    "vl_ens_schedule", "vl_ens_schedule_by_order", "vl_ens_commit", "vl_ens_steps", "vl_ens_begin",
+    "vl_ens_collect", "vl_run_state_write", "vl_mlp_dims", "vl_mlp_forward",
     "vl_mlp_partial_floats", "vl_mlp_backward", "vl_mlp_adam", "vl_closure_features", "vl_closure_apply",
     "vl_poisson_dg", "vl_axpby_interior",
 )
@@ -120,6 +121,9 @@ def _declare(lib):
     lib.vl_ens_schedule_by_order.argtypes = [vp, i32, ctypes.c_uint32]
     lib.vl_ens_commit.argtypes = [vp]
     lib.vl_ens_steps.argtypes = [vp, i32, vp]
+    lib.vl_ens_begin.argtypes = [vp, ctypes.c_int64, vp]
+    lib.vl_ens_collect.argtypes = [vp, i32, vp, vp]
+    lib.vl_run_state_write.argtypes = [vp, ctypes.POINTER(VlRunState), vp]
     f32, f64 = ctypes.c_float, ctypes.c_double
     pi32 = ctypes.POINTER(i32)
     lib.vl_mlp_dims.argtypes = [pi32, pi32, pi32, pi32, pi32]
@@ -168,5 +172,6 @@ def check(fn_name: str, code: int):
 
 
 def call(fn_name: str, *args):
-    lib = load()
-    check(fn_name, getattr(lib, fn_name)(*args))
+    code = getattr(_lib or load(), fn_name)(*args)
+    if code != VL_OK:
+        check(fn_name, code)

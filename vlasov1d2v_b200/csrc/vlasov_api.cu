@@ -984,6 +984,9 @@ int upload(P **dst, const void *src, size_t bytes) {
     return VL_OK;
 }
 
+// a host loop state, carried in the launch parameters
+static __global__ void run_state_kernel(vl_run_state *state, const vl_run_state host) { *state = host; }
+
 // The loop with the field solves inside the stage kernels: three launches a step, and one at the end
 // that closes the last step.
 int fused_steps(vl_ctx *c, void *f, void *sa, void *sb, double *E, double *phi, vl_run_state *state, void *workspace,
@@ -1467,6 +1470,12 @@ int vl_run_state_init(vl_ctx *c, vl_run_state *state, const double *E0, double f
     a.cap = cap;
     vl::scalars_kernel<<<1, vl::FIELD_THREADS, 0, as_stream(stream)>>>(a);
     return check_launch("scalars_kernel(init)");
+}
+
+int vl_run_state_write(vl_run_state *state, const vl_run_state *host, void *stream) {
+    if (!state || !host) return fail(VL_ERR_INVALID, "null argument");
+    run_state_kernel<<<1, 1, 0, as_stream(stream)>>>(state, *host);
+    return check_launch("run_state_kernel");
 }
 
 int vl_set_background_pairs(vl_ctx *c, const float *pairs) {

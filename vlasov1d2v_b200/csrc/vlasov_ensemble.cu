@@ -91,6 +91,35 @@ __host__ __device__ __forceinline__ void ens_stage_args(StageArgs &a, const EnsM
     }
 }
 
+// every member's loop state made ready for a batch, a thread each
+__global__ void ens_begin_kernel(const EnsMember *__restrict__ members, int count, int64_t max_steps) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    vl_run_state *st = const_cast<vl_run_state *>(members[i].a.state);
+    st->steps = 0;
+    st->max_steps = max_steps;
+    st->active_next = st->time < st->final_time && st->status == 0;
+}
+
+// results of a batch, a CTA per member: one copy to the host for the whole ensemble instead of a state and
+// three history rows a member (24 members: 2.6 ms of host work per call)
+__global__ void ens_collect_kernel(const EnsMember *__restrict__ members, int k, double *__restrict__ out) {
+    const vl_run_state *st = members[blockIdx.x].a.state;
+    double *row = out + (size_t)blockIdx.x * (2 + 3 * (size_t)k);
+    const int64_t steps = st->steps;
+    const int kept = (int)(steps < st->hist_capacity ? steps : st->hist_capacity);
+    if (threadIdx.x == 0) {
+        row[0] = (double)steps;
+        row[1] = (double)st->status;
+    }
+    for (int s = threadIdx.x; s < k; s += blockDim.x) {
+        const bool in = s < kept;
+        row[2 + s] = in && st->energy_hist ? st->energy_hist[s] : 0.0;
+        row[2 + k + s] = in && st->time_hist ? st->time_hist[s] : 0.0;
+        row[2 + 2 * k + s] = in && st->dt_hist ? st->dt_hist[s] : 0.0;
+    }
+}
+
 template <int N>
 struct EnsJC {
     // j values per thread so that NT / 32 warps cover the n rows
@@ -810,6 +839,24 @@ VL_API int vl_ens_schedule_by_order(vl_ens *E, int32_t items_per_cta, uint32_t n
 VL_API int vl_ens_commit(vl_ens *E) {
     if (!E) return efail(VL_ERR_INVALID, "null ensemble");
     return commit(E);
+}
+
+VL_API int vl_ens_begin(vl_ens *E, int64_t max_steps, void *stream) {
+    if (!E) return efail(VL_ERR_INVALID, "null ensemble");
+    if (E->dirty) return efail(VL_ERR_INVALID, "ensemble changed since the last vl_ens_commit");
+    const int count = (int)E->ctx.size();
+    vl::ens_begin_kernel<<<(count + 63) / 64, 64, 0, static_cast<cudaStream_t>(stream)>>>(E->d_members, count, max_steps);
+    VL_ECUDA(cudaGetLastError());
+    return VL_OK;
+}
+
+VL_API int vl_ens_collect(vl_ens *E, int32_t k, double *out, void *stream) {
+    if (!E || !out) return efail(VL_ERR_INVALID, "null argument");
+    if (k < 0) return efail(VL_ERR_INVALID, "k < 0");
+    if (E->dirty) return efail(VL_ERR_INVALID, "ensemble changed since the last vl_ens_commit");
+    vl::ens_collect_kernel<<<(int)E->ctx.size(), 128, 0, static_cast<cudaStream_t>(stream)>>>(E->d_members, k, out);
+    VL_ECUDA(cudaGetLastError());
+    return VL_OK;
 }
 
 VL_API int vl_ens_steps(vl_ens *E, int32_t nsteps, void *stream) {

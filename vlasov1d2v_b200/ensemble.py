@@ -190,29 +190,22 @@ class Ensemble:
         remaining = int(nsteps)
         while remaining > 0:
             k = min(self.batch, remaining)
-            for r, p in zip(self.runs, self.problems):
-                st = r.read_state()
-                st.steps = 0
-                st.max_steps = k
-                st.active_next = int(st.time < st.final_time and st.status == 0)
-                r.upload_state(st)
+            stream = _device.stream_handle()
+            _lib.call("vl_ens_begin", self.handle, k, stream)
             self.launch(k, use_graph)
-            for r, p in zip(self.runs, self.problems):
-                st = r.read_state()
-                if st.status != 0:
+            rows = torch.empty((len(self.runs), 2 + 3 * k), dtype=torch.float64, device=self.runs[0].f.device)
+            _lib.call("vl_ens_collect", self.handle, k, rows.data_ptr(), stream)
+            if k == remaining:   # the members' fields, enqueued before the host waits
+                fields = [r.fields() for r in self.runs]
+            for r, p, row in zip(self.runs, self.problems, rows.cpu().numpy()):
+                if row[1] != 0:
                     raise NonFiniteError("non-finite field or energy in an ensemble member")
-                h = r.hist[:, :int(st.steps)].cpu().numpy()
-                stp = p.stepper
-                for s in range(int(st.steps)):
-                    stp.time = float(h[1, s])
-                    stp.steps_counter += 1
-                    stp.time_array = np.append(stp.time_array, stp.time)
-                    stp.field_energy = np.append(stp.field_energy, h[0, s])
-                    stp.dt = float(h[2, s])
+                p.stepper.record(row[2:].reshape(3, k)[:, :r.cap], int(row[0]))
             remaining -= k
-        for r, p in zip(self.runs, self.problems):
-            p.elliptic.electric_field = _device.wrap(r.E.clone())
-            p.elliptic.potential = _device.wrap(r.phi.clone())
+        if int(nsteps) < 1:
+            fields = [r.fields() for r in self.runs]
+        for p, (E, phi) in zip(self.problems, fields):
+            p.elliptic.electric_field, p.elliptic.potential = E, phi
 
     def total_dof(self):
         return sum(r.ctx.nx * r.ctx.nu * r.ctx.nv * r.ctx.n ** 3 for r in self.runs)

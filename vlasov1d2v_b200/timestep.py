@@ -58,6 +58,9 @@ class NonFiniteError(FloatingPointError):
     """The device loop detected a non-finite density, field, energy or dt."""
 
 
+_HIST_OFFSET = (_lib.RUN_STATE_BYTES + 127) // 128 * 128   # histories behind the loop state
+
+
 class _Run:
     """Device buffers of one (distribution, grids, physics) loop set-up."""
 
@@ -69,8 +72,10 @@ class _Run:
         self.sb = torch.empty_like(f)
         self.E = torch.zeros((ctx.nx + 2, ctx.n), dtype=torch.float64, device=dev)
         self.phi = torch.zeros((ctx.nx, ctx.n), dtype=torch.float64, device=dev)
-        self.state = torch.zeros(_lib.RUN_STATE_BYTES, dtype=torch.uint8, device=dev)
-        self.hist = torch.zeros((3, hist_cap), dtype=torch.float64, device=dev)
+        # loop state and histories in one buffer: a batch's result is one device -> host copy
+        self.block = torch.zeros(_HIST_OFFSET + 24 * hist_cap, dtype=torch.uint8, device=dev)
+        self.state = self.block[:_lib.RUN_STATE_BYTES]
+        self.hist = self.block[_HIST_OFFSET:].view(torch.float64).view(3, hist_cap)
         self.cap = hist_cap
         self.graph = None
         self.graph_steps = 0
@@ -78,12 +83,21 @@ class _Run:
         self.background = None   # RHS tables of the FP32 background split, or None
 
     def upload_state(self, st: _lib.VlRunState):
-        host = torch.frombuffer(bytearray(bytes(st)), dtype=torch.uint8)
-        self.state.copy_(host, non_blocking=False)
+        _lib.call("vl_run_state_write", self.state.data_ptr(), st, _device.stream_handle())
 
     def read_state(self) -> _lib.VlRunState:
         raw = self.state.cpu().numpy().tobytes()
         return _lib.VlRunState.from_buffer_copy(raw)
+
+    def fields(self):
+        """Copies of the field and the potential."""
+        return _device.wrap(self.E.clone()), _device.wrap(self.phi.clone())
+
+    def read_batch(self):
+        """The loop state and the histories (energy, time, dt) on the host."""
+        raw = self.block.cpu().numpy()
+        st = _lib.VlRunState.from_buffer_copy(raw[:_lib.RUN_STATE_BYTES])
+        return st, raw[_HIST_OFFSET:].view(np.float64).reshape(3, self.cap)
 
     def sync_ghosts(self):
         self.ctx.sync_stage_ghosts(self.f, self.sa, self.sb)
@@ -214,6 +228,15 @@ class Stepper:
         self.field_energy = np.array(checkpoint["field_energy"], dtype=np.float64)
         self._resumed = True
 
+    def record(self, hist, steps):
+        """Append the histories (energy, time, dt rows) of ``steps`` steps."""
+        if steps > 0:
+            self.time = float(hist[1, steps - 1])
+            self.dt = float(hist[2, steps - 1])
+            self.steps_counter += steps
+            self.time_array = np.append(self.time_array, hist[1, :steps])
+            self.field_energy = np.append(self.field_energy, hist[0, :steps])
+
     def main_loop(self, distribution, basis, elliptic, grids, dg_flux, refs, save_file):
         t0 = timer.time()
         if getattr(self, "_resumed", False):
@@ -231,17 +254,16 @@ class Stepper:
             k = self.batch_steps
             run.launch(k, self.use_graph and batches > 0)
             batches += 1
-            st = run.read_state()
+            st, h = run.read_batch()
             new = int(st.steps)
             if new > 0:
-                h = run.hist[:, :new].cpu().numpy() if new <= run.cap else None
-                if h is None:
+                if new > run.cap:
                     raise RuntimeError("history ring overflow")
+                self.time_array = np.append(self.time_array, h[1, :new])
+                self.field_energy = np.append(self.field_energy, h[0, :new])
                 for s in range(new):
                     self.time = float(h[1, s])
                     self.steps_counter += 1
-                    self.time_array = np.append(self.time_array, self.time)
-                    self.field_energy = np.append(self.field_energy, h[0, s])
                     self.dt = float(h[2, s])
                     if self.time > self.write_counter * self.write_time:
                         self.write_counter += 1
@@ -280,24 +302,19 @@ class Stepper:
         saved_final, saved_verbose = self.final_time, self.verbose
         remaining = int(nsteps)
         run = self._run(distribution, elliptic, grids, refs)
+        fields = run.fields() if remaining <= 0 else None
         while remaining > 0:
             k = min(self.batch_steps, remaining)
             run.upload_state(self._host_state(run, float("inf"), k))
             run.launch(k, False)
-            st = run.read_state()
-            h = run.hist[:, :int(st.steps)].cpu().numpy()
-            for s in range(int(st.steps)):
-                self.time = float(h[1, s])
-                self.steps_counter += 1
-                self.time_array = np.append(self.time_array, self.time)
-                self.field_energy = np.append(self.field_energy, h[0, s])
-                self.dt = float(h[2, s])
+            fields = run.fields()   # enqueued before the host waits
+            st, h = run.read_batch()
+            self.record(h, int(st.steps))
             if st.status != 0:
                 raise NonFiniteError("non-finite field or energy detected")
             remaining -= int(st.steps)
         self.final_time, self.verbose = saved_final, saved_verbose
-        elliptic.electric_field = _device.wrap(run.E.clone())
-        elliptic.potential = _device.wrap(run.phi.clone())
+        elliptic.electric_field, elliptic.potential = fields
 
     def nonlinear_ssp_rk(self, distribution, basis, elliptic, grids, dg_flux, refs):
         """One nonlinear SSP-RK3 step (``main/timestep.py:141-187``): f advanced in place,
@@ -309,12 +326,12 @@ class Stepper:
         st.time = 0.0
         run.upload_state(st)
         run.launch(1, False)
+        fields = run.fields()   # enqueued before the host waits
         st = run.read_state()
         if st.status != 0:
             raise NonFiniteError("non-finite field or energy detected")
         self.dt = float(st.dt_next)
-        elliptic.electric_field = _device.wrap(run.E.clone())
-        elliptic.potential = _device.wrap(run.phi.clone())
+        elliptic.electric_field, elliptic.potential = fields
 
     def ssp_rk_update(self, distribution, basis, grids, elliptic, dg_flux, refs):
         """One step of the linear SSP-RK stepper of any order (``main/timestep.py:189-229``),
