@@ -1319,10 +1319,10 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
         c->fuse_field = c->d_ke != nullptr && one_wave && room >= vl::field_fuse_scratch(cfg->nx, n) &&
                         !(env && std::string(env) == "solve");
     }
-    // standalone moment: MOMENT_CTAS_PER_SM resident CTAs per SM, at most one per u element
-    int gm = (c->sm_count * vl::MOMENT_CTAS_PER_SM) / cfg->nx;
-    if (gm > cfg->nu) gm = cfg->nu;
-    if (gm < 1) gm = 1;
+    // standalone moment: a tile is one column per column thread
+    const int mcols = vl::MOMENT_THREADS / n * n;
+    const int gm = wave_grid((int)(((int64_t)cfg->nu * cfg->nv * n + mcols - 1) / mcols), cfg->nx,
+                             c->sm_count * vl::MOMENT_CTAS_PER_SM);
     c->moment_grid_g = gm;
     {
         const cudaError_t ee =
@@ -1400,7 +1400,7 @@ int vl_moment(vl_ctx *c, const void *f, double *rho, void *stream) {
     int rc = moment(c, f, c->d_moment, G, s);
     if (rc) return rc;
     const int nn = c->cfg.nx * c->cfg.n;
-    vl::moment_reduce_kernel<<<(nn + 255) / 256, 256, 0, s>>>(c->d_moment, rho, c->cfg.nx, G, c->cfg.n);
+    vl::moment_reduce_kernel<<<(nn + 63) / 64, 64, 0, s>>>(c->d_moment, rho, c->cfg.nx, G, c->cfg.n);
     return check_launch("moment_reduce_kernel");
 }
 
@@ -1417,7 +1417,7 @@ int vl_field_energy(vl_ctx *c, const double *E, double *energy, void *stream) {
     if (!c || !E || !energy) return fail(VL_ERR_INVALID, "null argument");
     vl::ScalarArgs a = scalar_args(c, E);
     a.energy = energy;
-    vl::scalars_kernel<<<1, vl::FIELD_THREADS, 0, as_stream(stream)>>>(a);
+    vl::scalars_kernel<<<1, vl::SCALAR_THREADS, 0, as_stream(stream)>>>(a);
     return check_launch("scalars_kernel");
 }
 
@@ -1425,7 +1425,7 @@ int vl_adapt_dt(vl_ctx *c, const double *E, double *dt, void *stream) {
     if (!c || !E || !dt) return fail(VL_ERR_INVALID, "null argument");
     vl::ScalarArgs a = scalar_args(c, E);
     a.dt = dt;
-    vl::scalars_kernel<<<1, vl::FIELD_THREADS, 0, as_stream(stream)>>>(a);
+    vl::scalars_kernel<<<1, vl::SCALAR_THREADS, 0, as_stream(stream)>>>(a);
     return check_launch("scalars_kernel");
 }
 
@@ -1468,7 +1468,7 @@ int vl_run_state_init(vl_ctx *c, vl_run_state *state, const double *E0, double f
     a.th = th;
     a.dh = dh;
     a.cap = cap;
-    vl::scalars_kernel<<<1, vl::FIELD_THREADS, 0, as_stream(stream)>>>(a);
+    vl::scalars_kernel<<<1, vl::SCALAR_THREADS, 0, as_stream(stream)>>>(a);
     return check_launch("scalars_kernel(init)");
 }
 

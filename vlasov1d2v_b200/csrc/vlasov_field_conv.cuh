@@ -36,17 +36,6 @@ __host__ __device__ constexpr size_t field_conv_smem(int nx, int n, bool phi) {
     return sizeof(double) * (size_t)(phi ? 2 : 1) * field_conv_elems(nx, n);
 }
 
-// compensated sum: the high part is one addition per term, the rounding errors are gathered beside it
-__device__ __forceinline__ dd dd_gather(dd a, dd b) {
-    const double s = a.hi + b.hi;
-    const double bp = s - a.hi;
-    return {s, ((a.hi - (s - bp)) + (b.hi - bp)) + (a.lo + b.lo)};
-}
-
-__device__ __forceinline__ dd dd_shfl_xor(dd v, int off) {
-    return {__shfl_xor_sync(0xffffffffu, v.hi, off), __shfl_xor_sync(0xffffffffu, v.lo, off)};
-}
-
 // KE and KP: 8 lanes share a value's sum over the modes (compensated; 40 us with one thread per value
 // at 16 elements of n = 8, 11 us now)
 static __global__ void __launch_bounds__(256) field_conv_table_kernel(double *KE, double *KP, const double2 *ell,

@@ -134,27 +134,22 @@ __device__ __forceinline__ dd dd_add(dd a, dd b) {
     return r;
 }
 
+// compensated sum: the high part is one addition per term, the rounding errors are gathered beside it
+// (dd_add renormalises each term: four more additions on the chain)
+__device__ __forceinline__ dd dd_gather(dd a, dd b) {
+    const double s = a.hi + b.hi;
+    const double bp = s - a.hi;
+    return {s, ((a.hi - (s - bp)) + (b.hi - bp)) + (a.lo + b.lo)};
+}
+
+__device__ __forceinline__ dd dd_shfl_xor(dd v, int off) {
+    return {__shfl_xor_sync(0xffffffffu, v.hi, off), __shfl_xor_sync(0xffffffffu, v.lo, off)};
+}
+
 __device__ __forceinline__ dd shfl_down_dd(dd v, int off) {
     dd r;
     r.hi = __shfl_down_sync(0xffffffffu, v.hi, off);
     r.lo = __shfl_down_sync(0xffffffffu, v.lo, off);
-    return r;
-}
-
-// ----------------------------------------------------------------------------------------------
-// standalone moment: grid (G, nx).  CTA (g, e) sums the interior u elements
-// [g nu / G, (g + 1) nu / G) of x slab e for every x node i and writes
-// out[(e G + g) n + i] -- the layout of the stage kernels' moment partials.
-// Columns go to threads with a stride that is a multiple of n, so each thread sees one v node
-// k and keeps its row of weights w_j w_k / (J_u J_v) in registers.
-// ----------------------------------------------------------------------------------------------
-// runtime-indexed read of a small register array (unrolled select)
-template <int N>
-__device__ __forceinline__ double acc_at(const double (&v)[N], int i) {
-    double r = v[0];
-#pragma unroll
-    for (int m = 1; m < N; ++m)
-        if (m == i) r = v[m];
     return r;
 }
 
@@ -179,6 +174,17 @@ struct MomentArgs {
     double qw[NMAX * NMAX];
 };
 
+// ----------------------------------------------------------------------------------------------
+// standalone moment: grid (G, nx).  CTA (g, e) sums its share of the nu nv velocity elements of x slab e
+// for every x node i and writes out[(e G + g) n + i] -- the layout of the stage kernels' moment partials.
+// A share is a run of columns (u element, v node) of the slab; columns go to threads with a stride that
+// is a multiple of n, so each thread sees one v node k and keeps its row of weights w_j w_k / (J_u J_v)
+// in registers.  Bound by HBM on large grids (with the reduction over CTAs, 32x50x50 n = 8: FP64 66 us with
+// shares of whole u elements, 56 now; FP32 45 -> 34; 64^3 n = 9 279 -> 237), by latency on small ones, where
+// the sums over the threads were most of the time: node by node, each five shuffles, two barriers and a
+// chain over the warps; now a warp per node over all threads' sums at once (16^3 n = 8 15.5 -> 5.9 us,
+// 16x20x20 n = 6 13.4 -> 6.0).
+// ----------------------------------------------------------------------------------------------
 constexpr int MOMENT_THREADS = 256;
 // 2 resident CTAs per SM leave 128 registers per thread, room for most of a column's n x n loads
 // in flight at once (at 4 CTAs, 64 registers, the loads issued a few at a time and the kernel ran
@@ -189,14 +195,16 @@ template <int N, typename T>
 __global__ void __launch_bounds__(MOMENT_THREADS, MOMENT_CTAS_PER_SM) moment_kernel(const MomentArgs a) {
     const T *__restrict__ f = static_cast<const T *>(a.f);
     constexpr int CT = (MOMENT_THREADS / N) * N;   // column threads (stride keeps k fixed)
+    constexpr int NW = MOMENT_THREADS / 32;
+    __shared__ double part[N][MOMENT_THREADS];
     const int g = blockIdx.x, Gn = gridDim.x, e = blockIdx.y;
     const int nu = a.nu, nv = a.nv;
     const int U = nu + 2, V = nv + 2;
     const int sJ = V * N, sA = sJ * N, sI = sA * U;
-    const size_t slab = (size_t)(e + 1) * ((size_t)sI * N);
-    const int a_lo = (int)(((long long)g * nu) / Gn), a_hi = (int)(((long long)(g + 1) * nu) / Gn);
-    const int tid = threadIdx.x;
-    const int ncol = nv * N;
+    const int ncol = nv * N, cells = nu * nv;
+    const int lo = (int)(((long long)g * cells) / Gn) * N, hi = (int)(((long long)(g + 1) * cells) / Gn) * N;
+    const T *const slab = f + (size_t)(e + 1) * ((size_t)sI * N) + sA + N;   // first interior column
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int k = tid % N;
     double w[N];
 #pragma unroll
@@ -205,23 +213,31 @@ __global__ void __launch_bounds__(MOMENT_THREADS, MOMENT_CTAS_PER_SM) moment_ker
 #pragma unroll
     for (int i = 0; i < N; ++i) acc[i] = 0.0;
     if (tid < CT) {
-        for (int au = a_lo; au < a_hi; ++au) {
-            const T *pa = f + slab + (size_t)(au + 1) * sA + N;   // interior columns start at N
-            for (int c = tid; c < ncol; c += CT) {
+        for (int q = lo + tid; q < hi; q += CT) {
+            const int au = q / ncol;
+            const T *pi = slab + (size_t)au * sA + (q - au * ncol);
+            // the row strides are opaque here: kept across columns, the offsets of the n x n rows take the
+            // registers that the loads in flight need (32x50x50 n = 8 100 us)
+            int si = sI, sj = sJ;
+            asm volatile("" : "+r"(si), "+r"(sj));
 #pragma unroll
-                for (int i = 0; i < N; ++i) {
-                    double s = 0.0;
+            for (int i = 0; i < N; ++i) {
+                double s = 0.0;
 #pragma unroll
-                    for (int j = 0; j < N; ++j) s = fma(w[j], (double)pa[(size_t)i * sI + j * sJ + c], s);
-                    acc[i] += s;
-                }
+                for (int j = 0; j < N; ++j) s = fma(w[j], (double)pi[i * si + j * sj], s);
+                acc[i] += s;
             }
         }
     }
-    __shared__ dd red[MOMENT_THREADS / 32];
-    for (int i = 0; i < N; ++i) {
-        const double tot = block_sum_dd_rt(acc_at(acc, i), 0.0, red);
-        if (tid == 0) a.out[((size_t)e * Gn + g) * N + i] = tot;
+#pragma unroll
+    for (int i = 0; i < N; ++i) part[i][tid] = acc[i];
+    __syncthreads();
+    for (int i = warp; i < N; i += NW) {
+        dd s = {part[i][lane], 0.0};
+#pragma unroll
+        for (int m = 1; m < NW; ++m) s = dd_gather(s, dd{part[i][lane + 32 * m], 0.0});
+        for (int off = 16; off > 0; off >>= 1) s = dd_gather(s, dd_shfl_xor(s, off));
+        if (lane == 0) a.out[((size_t)e * Gn + g) * N + i] = s.hi + s.lo;
     }
 }
 
@@ -231,8 +247,10 @@ static __global__ void moment_reduce_kernel(const double *__restrict__ partials,
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= nx * n) return;
     const int e = p / n, i = p - e * n;
+    const double *src = partials + (size_t)e * G * n + i;
     dd s = {0.0, 0.0};
-    for (int g = 0; g < G; ++g) s = dd_add(s, dd{partials[((size_t)e * G + g) * n + i], 0.0});
+#pragma unroll 8
+    for (int g = 0; g < G; ++g) s = dd_gather(s, dd{src[(size_t)g * n], 0.0});
     rho[p] = s.hi + s.lo;
 }
 
@@ -267,7 +285,7 @@ struct FieldArgs {
     const double *KE, *KP;
 };
 
-constexpr int FIELD_THREADS = 1024;            // threads of the single-CTA scalar kernel
+constexpr int SCALAR_THREADS = 256;           // threads of the single-CTA scalar kernel
 constexpr int FIELD_MAX_NODES = 64 * NMAX;    // nx * n capacity of the shared buffers
 constexpr int FIELD_MAX_MODES = 2 * 160 + 1;  // M capacity
 
@@ -317,25 +335,40 @@ struct ScalarArgs {
     int cap;
 };
 
-static __global__ void __launch_bounds__(FIELD_THREADS) scalars_kernel(const ScalarArgs a) {
-    __shared__ dd s_red[FIELD_THREADS / 32];
-    __shared__ double s_max[FIELD_THREADS / 32];
+// Latency: a few terms a thread, then one sum and one maximum over the CTA, both in one pass (two serial
+// passes over 32 warps' parts took 8.3 us, this 2.4)
+static __global__ void __launch_bounds__(SCALAR_THREADS) scalars_kernel(const ScalarArgs a) {
+    constexpr int NW = SCALAR_THREADS / 32;
+    __shared__ dd s_sum[NW];
+    __shared__ double s_max[NW];
     const int nn = a.nx * a.n;
-    double esq = 0.0, esqc = 0.0, emax = 0.0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    dd esq = {0.0, 0.0};
+    double emax = 0.0;
     // energy over the interior rows E[1:-1]; max |a E| over all rows incl. ghosts
-    for (int p = threadIdx.x; p < nn + 2 * a.n; p += blockDim.x) {
+    for (int p = threadIdx.x; p < nn + 2 * a.n; p += SCALAR_THREADS) {
         const double er = a.E[p];
         emax = fmax(emax, fabs(a.accel * er));
-        if (p >= a.n && p < nn + a.n) {
-            const double v = a.xw[p % a.n] * (er * er);
-            const double t = esq + v;
-            esqc += (fabs(esq) >= fabs(v)) ? ((esq - t) + v) : ((v - t) + esq);
-            esq = t;
-        }
+        if (p >= a.n && p < nn + a.n) esq = dd_gather(esq, dd{a.xw[p % a.n] * (er * er), 0.0});
     }
-    const double energy = 0.5 * block_sum_dd(esq, esqc, s_red);
-    const double maxE = block_max(emax, s_max);
+    for (int off = 16; off > 0; off >>= 1) {
+        esq = dd_gather(esq, dd_shfl_xor(esq, off));
+        emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, off));
+    }
+    if (lane == 0) {
+        s_sum[warp] = esq;
+        s_max[warp] = emax;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
+        dd t = s_sum[0];
+        double maxE = s_max[0];
+#pragma unroll
+        for (int w = 1; w < NW; ++w) {
+            t = dd_gather(t, s_sum[w]);
+            maxE = fmax(maxE, s_max[w]);
+        }
+        const double energy = 0.5 * (t.hi + t.lo);
         const double ab = a.accel * a.bfield;
         const double s0 = fabs(a.umax);
         const double s1 = fabs(maxE + fabs(ab * a.vmax));

@@ -358,8 +358,7 @@ stage_f32_kernel(const StageArgs a, const __grid_constant__ F32Tables tb, const 
     // half-warp that holds node g (its four elements and column pairs)
     dd v = two_sum(tb.wv[k0] * mk0, tb.wv[k1] * mk1);
 #pragma unroll
-    for (int off = 1; off < 16; off <<= 1)
-        v = dd_add(v, dd{__shfl_xor_sync(0xffffffffu, v.hi, off), __shfl_xor_sync(0xffffffffu, v.lo, off)});
+    for (int off = 1; off < 16; off <<= 1) v = dd_gather(v, dd_shfl_xor(v, off));
     if ((lane & 15) == 0) sRed[g] = v;
     __syncthreads();
     if (tid < N) a.partials[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * N + tid] = sRed[tid].hi + sRed[tid].lo;

@@ -462,14 +462,14 @@ stage_frag_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
     if (a.partials == nullptr) return;
     // moment partial of x node g: sum over the thread's columns, the quad, the warps
     dd v = two_sum(tb.wv[2 * t] * mk0, tb.wv[2 * t + 1] * mk1);
-    v = dd_add(v, dd{__shfl_xor_sync(0xffffffffu, v.hi, 1), __shfl_xor_sync(0xffffffffu, v.lo, 1)});
-    v = dd_add(v, dd{__shfl_xor_sync(0xffffffffu, v.hi, 2), __shfl_xor_sync(0xffffffffu, v.lo, 2)});
+    v = dd_gather(v, dd_shfl_xor(v, 1));
+    v = dd_gather(v, dd_shfl_xor(v, 2));
     if (t == 0) sRed[wid][g] = v;
     __syncthreads();
     if (tid < N) {
         dd s = sRed[0][tid];
 #pragma unroll
-        for (int ww = 1; ww < EPT * G::JS; ++ww) s = dd_add(s, sRed[ww][tid]);
+        for (int ww = 1; ww < EPT * G::JS; ++ww) s = dd_gather(s, sRed[ww][tid]);
         a.partials[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * N + tid] = s.hi + s.lo;
     }
     (void)NT;

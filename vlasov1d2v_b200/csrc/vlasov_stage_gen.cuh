@@ -843,7 +843,7 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
     if (tid < N) {
         dd s = {0.0, 0.0};
         for (int bb = 0; bb < EPT; ++bb)
-            for (int pp = 0; pp < P; ++pp) s = dd_add(s, sRed[(bb * N + tid) * P + pp]);
+            for (int pp = 0; pp < P; ++pp) s = dd_gather(s, sRed[(bb * N + tid) * P + pp]);
         a.partials[((size_t)e * G + g) * N + tid] = s.hi + s.lo;
     }
     (void)NT;

@@ -459,8 +459,8 @@ stage_line_kernel(const StageArgs a, const __grid_constant__ LineTables<N, T> tb
     const int lane = tid & 31;
     for (int i = tid >> 5; i < N; i += G::NW) {
         dd s = {0.0, 0.0};
-        for (int cc = lane; cc < COLS; cc += 32) s = dd_add(s, dd{sRed[i * COLS + cc], 0.0});
-        for (int off = 16; off > 0; off >>= 1) s = dd_add(s, shfl_down_dd(s, off));
+        for (int cc = lane; cc < COLS; cc += 32) s = dd_gather(s, dd{sRed[i * COLS + cc], 0.0});
+        for (int off = 16; off > 0; off >>= 1) s = dd_gather(s, dd_shfl_xor(s, off));
         if (lane == 0) a.partials[((size_t)e * GX + blockIdx.x) * N + i] = s.hi + s.lo;
     }
 }
