@@ -105,6 +105,14 @@ cudaError_t launch(const vl_ctx *c, void (*kernel)(K...), dim3 grid, dim3 block,
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+template <typename... K, typename... A>
+cudaError_t stage_launch(const vl::StageArgs &a, void (*kernel)(vl::StageArgs, K...), dim3 grid, int threads,
+                         size_t smem, cudaStream_t s, const A &...args) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = vl::stage_config(a, grid, threads, smem, s, &attr);
+    return cudaLaunchKernelEx(&cfg, kernel, a, args...);
+}
+
 // 5-D view of the ghost-inclusive state: (v node, j, a, i, e), innermost first
 template <int N, typename T>
 int state_map(vl_ctx *c, const void *ptr, int which, CUtensorMap *out) {
@@ -421,13 +429,12 @@ int launch_stage_t(vl_ctx *c, const vl::StageArgs &a0, cudaStream_t s) {
                 const vl::F32Tables &ft = f32_tables(c);
                 // background split: 0 none, 1 two tables, 2 the interleaved pair table
                 const int bg = a.bg_rb == nullptr ? 0 : (c->bg_pair != nullptr ? 2 : 1);
-                const dim3 blk(G::THREADS);
                 const size_t sm = G::smem_bytes();
                 auto go = [&](auto kc) {
                     constexpr int K = decltype(kc)::value;
-                    if (bg == 2) return launch(c, vl::stage_f32_kernel<K, 2>, grid, blk, sm, s, a, ft, maps);
-                    if (bg == 1) return launch(c, vl::stage_f32_kernel<K, 1>, grid, blk, sm, s, a, ft, maps);
-                    return launch(c, vl::stage_f32_kernel<K, 0>, grid, blk, sm, s, a, ft, maps);
+                    if (bg == 2) return stage_launch(a, vl::stage_f32_kernel<K, 2>, grid, G::THREADS, sm, s, ft, maps);
+                    if (bg == 1) return stage_launch(a, vl::stage_f32_kernel<K, 1>, grid, G::THREADS, sm, s, ft, maps);
+                    return stage_launch(a, vl::stage_f32_kernel<K, 0>, grid, G::THREADS, sm, s, ft, maps);
                 };
                 cudaError_t le;
                 switch (a.kind) {
@@ -447,16 +454,16 @@ int launch_stage_t(vl_ctx *c, const vl::StageArgs &a0, cudaStream_t s) {
                 // without it (3 CTAs per SM)
                 // (one instantiation per stage kind: no per-row branches on it)
                 if (a.kind == vl::KIND_COMBINE)
-                    return check_launch(launch(c, vl::stage_frag_kernel<T, true, vl::KIND_COMBINE>, grid,
-                                               dim3(G::THREADS), G::smem_bytes(), s, a, tb, maps),
+                    return check_launch(stage_launch(a, vl::stage_frag_kernel<T, true, vl::KIND_COMBINE>, grid,
+                                                     G::THREADS, G::smem_bytes(), s, tb, maps),
                                         "stage_frag_kernel");
                 using G1 = vl::FragGeom<T, false>;
                 if (a.kind == vl::KIND_EULER)
-                    return check_launch(launch(c, vl::stage_frag_kernel<T, false, vl::KIND_EULER>, grid,
-                                               dim3(G1::THREADS), G1::smem_bytes(), s, a, tb, maps),
+                    return check_launch(stage_launch(a, vl::stage_frag_kernel<T, false, vl::KIND_EULER>, grid,
+                                                     G1::THREADS, G1::smem_bytes(), s, tb, maps),
                                         "stage_frag_kernel");
-                return check_launch(launch(c, vl::stage_frag_kernel<T, false, vl::KIND_RHS>, grid, dim3(G1::THREADS),
-                                           G1::smem_bytes(), s, a, tb, maps),
+                return check_launch(stage_launch(a, vl::stage_frag_kernel<T, false, vl::KIND_RHS>, grid, G1::THREADS,
+                                                 G1::smem_bytes(), s, tb, maps),
                                     "stage_frag_kernel");
             }
         }
@@ -1001,6 +1008,7 @@ int fused_steps(vl_ctx *c, void *f, void *sa, void *sb, double *E, double *phi, 
     vl::StageArgs st = stage_args(c);
     st.err = &state->status;
     st.xhalo = VL_XHALO_PERIODIC;
+    st.pdl = 1;
     vl::FieldFuse &ff = st.ff;
     ff.KE = c->d_ke;
     ff.KP = c->d_kp;

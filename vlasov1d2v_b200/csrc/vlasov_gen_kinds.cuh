@@ -21,12 +21,8 @@ template <typename T, int N, bool PAIR, int K, int B, bool FUSE = false>
 cudaError_t launch_one(dim3 grid, size_t smem, cudaStream_t s, const StageArgs &a, const StageTables<T> &tb,
                        const GenMaps &maps) {
     constexpr int THREADS = PAIR ? GenPairGeom<N, T>::THREADS : GenTmaGeom<N, T>::THREADS;
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = stage_config(a, grid, THREADS, smem, s, &attr);
     return cudaLaunchKernelEx(&cfg, kernel<T, N, PAIR, K, B, FUSE>(), a, tb, maps);
 }
 

@@ -30,16 +30,16 @@ cudaError_t launch(const StageArgs &a0, const LineCoef &lc, dim3 grid, cudaStrea
     StageArgs a = a0;
     a.never = -1;
     const LineTables<N, T> tb = tables<N, T>(lc);
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = stage_config(a, grid, G::THREADS, G::smem_bytes(), s, &attr);
     auto go = [&](auto kc) {
         constexpr int K = decltype(kc)::value;
         if constexpr (sizeof(T) == 4) {
             if (a.bg_rb != nullptr) {
-                stage_line_kernel<N, T, K, 1><<<grid, G::THREADS, G::smem_bytes(), s>>>(a, tb);
-                return cudaGetLastError();
+                return cudaLaunchKernelEx(&cfg, &stage_line_kernel<N, T, K, 1>, a, tb);
             }
         }
-        stage_line_kernel<N, T, K, 0><<<grid, G::THREADS, G::smem_bytes(), s>>>(a, tb);
-        return cudaGetLastError();
+        return cudaLaunchKernelEx(&cfg, &stage_line_kernel<N, T, K, 0>, a, tb);
     };
     if (a.kind == KIND_EULER) return go(std::integral_constant<int, KIND_EULER>{});
     if (a.kind == KIND_COMBINE) return go(std::integral_constant<int, KIND_COMBINE>{});

@@ -64,7 +64,6 @@ stage_f32_kernel(const StageArgs a, const __grid_constant__ F32Tables tb, const 
     constexpr int N = G::N, P = G::P, W = G::W, PS = G::PS, WF = G::WF, PSF = G::PSF;
     constexpr int COLS = G::COLS, EPT = G::EPT;
     static_assert(G::THREADS == 128 && EPT == 4, "four warps of two x nodes each");
-    if (a.state != nullptr && a.state->active == 0) return;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(
@@ -113,6 +112,7 @@ stage_f32_kernel(const StageArgs a, const __grid_constant__ F32Tables tb, const 
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    if (!stage_gate(a)) return;
 
     auto stage_ptr = [&](int s) { return base + (size_t)s * G::STAGE_B; };
     auto issue = [&](int s, int q) {

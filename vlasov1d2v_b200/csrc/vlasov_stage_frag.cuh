@@ -129,7 +129,6 @@ stage_frag_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
     using V2 = typename Pair<T>::V;
     constexpr int N = G::N, P = G::P, W = G::W, PS = G::PS, WF = G::WF, PSF = G::PSF;
     constexpr int COLS = G::COLS, EPT = G::EPT, NT = G::THREADS;
-    if (a.state != nullptr && a.state->active == 0) return;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(
@@ -176,6 +175,7 @@ stage_frag_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    if (!stage_gate(a)) return;
 
     auto stage_ptr = [&](int s) { return base + (size_t)s * G::STAGE_B; };
     auto issue = [&](int s, int q) {

@@ -395,6 +395,7 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncthreads();
+        if (!stage_gate(a)) return;
     }
     auto stage_ptr = [&](int s) { return smem + (size_t)s * S_STAGE; };
     // one row of ncol tile columns: global run -> slot layout
@@ -867,7 +868,6 @@ template <int N, typename T, int KT = -1, int BT = -1, bool FUSE = false>
 __global__ void __launch_bounds__(GenTmaGeom<N, T>::THREADS, GenTmaGeom<N, T>::MINB)
 stage_gen_tma_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
                      const __grid_constant__ GenMaps maps) {
-    if (a.state != nullptr && a.state->active == 0) return;
     extern __shared__ __align__(16) unsigned char gen_smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(gen_smem_raw) + 127) & ~(uintptr_t)127);
@@ -880,7 +880,6 @@ template <int N, typename T, int KT = -1, int BT = -1, bool FUSE = false>
 __global__ void __launch_bounds__(GenPairGeom<N, T>::THREADS, GenPairGeom<N, T>::MINB)
 stage_gen_pair_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
                       const __grid_constant__ GenMaps maps) {
-    if (a.state != nullptr && a.state->active == 0) return;
     extern __shared__ __align__(16) unsigned char gen_smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(gen_smem_raw) + 127) & ~(uintptr_t)127);

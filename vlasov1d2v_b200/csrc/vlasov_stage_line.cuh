@@ -194,7 +194,6 @@ stage_line_kernel(const StageArgs a, const __grid_constant__ LineTables<N, T> tb
     constexpr int EPT = G::EPT, COLS = G::COLS, W = G::W, L = G::L, NN = N * N;
     constexpr uint32_t ES = sizeof(T);
     static_assert(BG == 0 || sizeof(T) == 4, "the background split is a form of FP32 states");
-    if (a.state != nullptr && a.state->active == 0) return;
 
     extern __shared__ __align__(128) unsigned char line_smem[];
     T *const sTile = reinterpret_cast<T *>(line_smem);   // two tile buffers
@@ -287,6 +286,7 @@ stage_line_kernel(const StageArgs a, const __grid_constant__ LineTables<N, T> tb
     for (int s = 0; s < L; ++s) mk[s] = 0.0;
 
     int cur = 0;
+    if (!stage_gate(a)) return;
     if (au < nu) load_tile(au, bt);
     if (KIND != KIND_RHS && a.ff.mode != FUSE_NONE) {
         // E at this x element while the first tile travels; the tile buffers are the scratch
