@@ -113,10 +113,11 @@ cudaError_t stage_launch(const vl::StageArgs &a, void (*kernel)(vl::StageArgs, K
     return cudaLaunchKernelEx(&cfg, kernel, a, args...);
 }
 
-// 5-D view of the ghost-inclusive state: (v node, j, a, i, e), innermost first
+// 5-D view of the ghost-inclusive state: (v node, j, a, i, e), innermost first.  which: 6 = tile, 7 = f^n
+// tile, 1 = x face, 2 = u face of the n = 8 kernels
 template <int N, typename T>
 int state_map(vl_ctx *c, const void *ptr, int which, CUtensorMap *out) {
-    using G = vl::TmaGeom<N, T>;
+    using F = vl::FragGeom<T>;
     auto key = std::make_pair(ptr, which);
     auto it = c->maps.find(key);
     if (it != c->maps.end()) {
@@ -130,19 +131,13 @@ int state_map(vl_ctx *c, const void *ptr, int which, CUtensorMap *out) {
     cuuint64_t dims[5] = {V * N, (cuuint64_t)N, U, (cuuint64_t)N, X};
     cuuint64_t strides[4] = {V * N * es, V * N * N * es, V * N * N * U * es, V * N * N * U * N * es};
     cuuint32_t box[5];
-    using F = vl::FragGeom<T>;
     switch (which) {
-        // fragment kernel tiles: one zero-filled row past the j extent pads the plane stride
+        // tiles: one zero-filled row past the j extent pads the plane stride
         case 6: box[0] = F::W; box[1] = F::ROWS; box[2] = 1; box[3] = N; box[4] = 1; break;
         case 7: box[0] = F::WF; box[1] = F::ROWS; box[2] = 1; box[3] = N; box[4] = 1; break;
-        case 0: case 5: box[0] = G::W; box[1] = N; box[2] = 1; box[3] = N; box[4] = 1; break;
-        case 1: box[0] = G::COLS; box[1] = N; box[2] = 1; box[3] = 1; box[4] = 1; break;
-        case 2: box[0] = G::COLS; box[1] = 1; box[2] = 1; box[3] = N; box[4] = 1; break;
-        default: box[0] = G::COLS; box[1] = N; box[2] = 1; box[3] = N; box[4] = 1; break;
+        case 1: box[0] = F::COLS; box[1] = N; box[2] = 1; box[3] = 1; box[4] = 1; break;
+        default: box[0] = F::COLS; box[1] = 1; box[2] = 1; box[3] = N; box[4] = 1; break;   // 2
     }
-    // output tiles: the v extent ends after the last interior element, so stores of a ragged
-    // last tile are clipped before the v ghost element
-    if (which == 4) dims[0] = (cuuint64_t)(c->cfg.nv + 1) * N;
     cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     CUtensorMap m;
     CUresult r = enc(&m, sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5,
@@ -522,20 +517,6 @@ int launch_stage_t(vl_ctx *c, const vl::StageArgs &a0, cudaStream_t s) {
         return check_launch(launch(c, vl::stage_gen_kernel<N, T>, grid, dim3(G::THREADS), G::smem_bytes(), s, a, tb),
                             "stage_gen_kernel");
     }
-    if constexpr (vl::TmaGeom<N, T>::SUPPORTED) {
-        if (c->use_tma) {
-            using G = vl::TmaGeom<N, T>;
-            vl::TmaMaps maps;
-            int rc;
-            if ((rc = state_map<N, T>(c, a.in, 0, &maps.in_tile))) return rc;
-            if ((rc = state_map<N, T>(c, a.in, 1, &maps.in_xface))) return rc;
-            if ((rc = state_map<N, T>(c, a.in, 2, &maps.in_uface))) return rc;
-            if ((rc = state_map<N, T>(c, a.fn ? a.fn : a.in, 3, &maps.fn_tile))) return rc;
-            return check_launch(
-                launch(c, vl::stage_tma_kernel<N, T>, grid, dim3(G::THREADS), G::smem_bytes(), s, a, tb, maps),
-                "stage_tma_kernel");
-        }
-    }
     using G = vl::PencilGeom<N, T>;
     return check_launch(launch(c, vl::stage_pencil_kernel<N, T>, grid, dim3(G::THREADS), G::smem_bytes(), s, a, tb),
                         "stage_pencil_kernel");
@@ -580,7 +561,7 @@ int stage(vl_ctx *c, const vl::StageArgs &a, cudaStream_t s) {
 }
 
 template <int N, typename T>
-int stage_occupancy_t(bool tma, bool frag, bool gen, bool gtma, bool gpair) {
+int stage_occupancy_t(bool frag, bool gen, bool gtma, bool gpair) {
     int blocks = 0;
     if constexpr (sizeof(T) == 4) {
         if (gen && gpair) {
@@ -647,18 +628,6 @@ int stage_occupancy_t(bool tma, bool frag, bool gen, bool gtma, bool gpair) {
             return blocks > 0 ? blocks : 1;
         }
     }
-    if constexpr (vl::TmaGeom<N, T>::SUPPORTED) {
-        if (tma) {
-            using G = vl::TmaGeom<N, T>;
-            const size_t smem = G::smem_bytes();
-            cudaFuncSetAttribute(vl::stage_tma_kernel<N, T>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, vl::stage_tma_kernel<N, T>,
-                                                              G::THREADS, smem) != cudaSuccess)
-                return 1;
-            return blocks > 0 ? blocks : 1;
-        }
-    }
     using G = vl::PencilGeom<N, T>;
     const size_t smem = G::smem_bytes();
     cudaFuncSetAttribute(vl::stage_pencil_kernel<N, T>,
@@ -686,27 +655,19 @@ int frag_nofn_occupancy() {
     return blocks > 0 ? blocks : 1;
 }
 
-template <int N, typename T>
-bool tma_supported_t(const vl_config &g) {
-    if constexpr (vl::TmaGeom<N, T>::SUPPORTED) {
-        return ((size_t)(g.nv + 2) * N * sizeof(T)) % 16 == 0;
-    }
-    return false;
-}
-
 template <typename T>
-int stage_occupancy(int n, bool tma, bool frag, bool gen, bool gtma, bool gpair) {
+int stage_occupancy(int n, bool frag, bool gen, bool gtma, bool gpair) {
     switch (n) {
-        case 1: return stage_occupancy_t<1, T>(tma, frag, gen, gtma, gpair);
-        case 2: return stage_occupancy_t<2, T>(tma, frag, gen, gtma, gpair);
-        case 3: return stage_occupancy_t<3, T>(tma, frag, gen, gtma, gpair);
-        case 4: return stage_occupancy_t<4, T>(tma, frag, gen, gtma, gpair);
-        case 5: return stage_occupancy_t<5, T>(tma, frag, gen, gtma, gpair);
-        case 6: return stage_occupancy_t<6, T>(tma, frag, gen, gtma, gpair);
-        case 7: return stage_occupancy_t<7, T>(tma, frag, gen, gtma, gpair);
-        case 8: return stage_occupancy_t<8, T>(tma, frag, gen, gtma, gpair);
-        case 9: return stage_occupancy_t<9, T>(tma, frag, gen, gtma, gpair);
-        case 10: return stage_occupancy_t<10, T>(tma, frag, gen, gtma, gpair);
+        case 1: return stage_occupancy_t<1, T>(frag, gen, gtma, gpair);
+        case 2: return stage_occupancy_t<2, T>(frag, gen, gtma, gpair);
+        case 3: return stage_occupancy_t<3, T>(frag, gen, gtma, gpair);
+        case 4: return stage_occupancy_t<4, T>(frag, gen, gtma, gpair);
+        case 5: return stage_occupancy_t<5, T>(frag, gen, gtma, gpair);
+        case 6: return stage_occupancy_t<6, T>(frag, gen, gtma, gpair);
+        case 7: return stage_occupancy_t<7, T>(frag, gen, gtma, gpair);
+        case 8: return stage_occupancy_t<8, T>(frag, gen, gtma, gpair);
+        case 9: return stage_occupancy_t<9, T>(frag, gen, gtma, gpair);
+        case 10: return stage_occupancy_t<10, T>(frag, gen, gtma, gpair);
         default: return 1;
     }
 }
@@ -753,18 +714,7 @@ int gen_ept(int n) {
     }
 }
 
-template <typename T>
-bool tma_supported(const vl_config &g) {
-    switch (g.n) {
-        case 2: return tma_supported_t<2, T>(g);
-        case 4: return tma_supported_t<4, T>(g);
-        case 8: return tma_supported_t<8, T>(g);
-        default: return false;
-    }
-}
-
-// v elements per tile of the stage kernel
-// v elements per stage tile: 32 / n for the pencil, TMA and fragment kernels (4 at n = 8)
+// v elements per stage tile: 32 / n for the pencil and n = 8 kernels
 int stage_epw(const vl_ctx *c) {
     if (c->stage_kernel == VL_STAGE_GEN)
         return c->cfg.precision == VL_FP64 ? gen_ept<double>(c->cfg.n) : gen_ept<float>(c->cfg.n);
@@ -1215,14 +1165,11 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
         ee = cudaMemset(c->d_err, 0, sizeof(int));
         if (ee != cudaSuccess) return cleanup(cuda_fail(ee, "cudaMemset(err)"));
     }
-    c->use_tma = (cfg->precision == VL_FP64 ? tma_supported<double>(*cfg) : tma_supported<float>(*cfg)) &&
-                 encode_fn() != nullptr;
+    c->use_frag = n == 8 && encode_fn() != nullptr;
     {
         const char *env = getenv("VLASOV1D2V_NO_TMA");
-        if (env && env[0] == '1') c->use_tma = false;
+        if (env && env[0] == '1') c->use_frag = false;
     }
-    // CTAs per x element: fill the device (resident CTAs x SMs), at most one per tile
-    c->use_frag = c->use_tma && n == 8;
     {
         const char *env = getenv("VLASOV1D2V_NO_FRAG");
         if (env && env[0] == '1') c->use_frag = false;
@@ -1234,8 +1181,7 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
     //     combination stage against 119 / 147 in the generic kernel's cp.async form; on 16-byte rows the
     //     TMA form is faster: 83 / 89 against 88 / 121 us at 32^3)
     //   FP32, orders 2 to 6: the generic kernel's TMA forms where the rows allow them (n = 6 at 32x62x62
-    //     91 / 100 us against 97 / 116 in the line form, n = 4 26 / 28 against 27 / 31 and 39 / 46 in the
-    //     order-4 TMA kernel, n = 2 at 64x128x128 31 / 33 against 44 / 49)
+    //     91 / 100 us against 97 / 116 in the line form, n = 4 26 / 28 against 27 / 31, n = 2 at 64x128x128 31 / 33 against 44 / 49)
     //   FP32, other orders and rows: the line form (64^3, n = 9: 703 / 865 us against 870 / 912 in the
     //     generic kernel's paired-row TMA form; n = 7 at 32x62x62 151 / 179 against 179 / 188 in its TMA
     //     form, at 24x31x33 32 / 40 against 56 / 63 in the register-pencil kernel)
@@ -1256,12 +1202,11 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
     const bool tma_better = cfg->precision == VL_FP64 ? tma64 : (gen_tma32 || gen_pair32) && n >= 2 && n <= 6;
     // the forms without the line kernel (they also say how the entry points want buffers aligned)
     const int general = cfg->precision == VL_FP64     ? VL_STAGE_GEN
-                        : c->use_tma                  ? VL_STAGE_TMA
                         : (gen_tma32 || gen_pair32)   ? VL_STAGE_GEN
                                                       : VL_STAGE_PENCIL;
-    c->state_align = (cfg->precision == VL_FP64 ? tma64 : general != VL_STAGE_PENCIL) ? 16
-                     : cfg->precision == VL_FP64                                       ? 8
-                                                                                       : 4;
+    c->state_align = c->use_frag || (cfg->precision == VL_FP64 ? tma64 : general != VL_STAGE_PENCIL) ? 16
+                     : cfg->precision == VL_FP64                                                      ? 8
+                                                                                                      : 4;
     c->stage_kernel = c->use_frag                                      ? VL_STAGE_FRAG
                       : tma_better                                     ? VL_STAGE_GEN
                       : line_ok                                        ? VL_STAGE_LINE
@@ -1276,15 +1221,14 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
             else if (k == "line" && line_ok) c->stage_kernel = VL_STAGE_LINE;
         }
         c->use_frag = c->stage_kernel == VL_STAGE_FRAG;
-        if (c->stage_kernel != VL_STAGE_TMA && c->stage_kernel != VL_STAGE_FRAG) c->use_tma = false;
     }
     const bool gen = c->stage_kernel == VL_STAGE_GEN;
     // generic kernel in its TMA form: FP64 rows of a 16-byte multiple (V n even), FP32 as above
     c->gen_tma = gen && (cfg->precision == VL_FP64 ? tma64 : gen_tma32);
     c->gen_pair = gen && !c->gen_tma && gen_pair32;
     const int occ = cfg->precision == VL_FP64
-                        ? stage_occupancy<double>(n, c->use_tma, c->use_frag, gen, c->gen_tma, false)
-                        : stage_occupancy<float>(n, c->use_tma, c->use_frag, gen, c->gen_tma, c->gen_pair);
+                        ? stage_occupancy<double>(n, c->use_frag, gen, c->gen_tma, false)
+                        : stage_occupancy<float>(n, c->use_frag, gen, c->gen_tma, c->gen_pair);
     const int bt = stage_epw(c);
     const int tiles = cfg->nu * ((cfg->nv + bt - 1) / bt);
     auto grid_for = [&](int o) { return wave_grid(tiles, cfg->nx, c->sm_count * o); };

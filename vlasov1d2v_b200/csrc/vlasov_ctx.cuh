@@ -12,7 +12,7 @@
 #include "vlasov_kernels.cuh"
 #include "vlasov_stage_f32.cuh"
 
-enum vl_stage_kernel { VL_STAGE_PENCIL = 0, VL_STAGE_TMA = 1, VL_STAGE_FRAG = 2, VL_STAGE_GEN = 3, VL_STAGE_LINE = 4 };
+enum vl_stage_kernel { VL_STAGE_PENCIL = 0, VL_STAGE_FRAG = 2, VL_STAGE_GEN = 3, VL_STAGE_LINE = 4 };
 
 struct vl_ctx {
     vl_config cfg;      // scalars (pointer members cleared)
@@ -42,7 +42,6 @@ struct vl_ctx {
     double *d_tables = nullptr;   // up [n n], xi [n 2], qw [n n]
     double *d_moment = nullptr;   // moment partials of vl_moment [nx][moment_grid_g][n]
     int *d_err = nullptr;         // device error word of operators run without a loop state
-    bool use_tma = false;         // stage kernel: TMA-pipelined form (aligned orders)
     bool use_frag = false;        // n = 8: quad-fragment stage kernel (tensor cores in FP64)
     int stage_kernel = VL_STAGE_GEN;   // which stage kernel the launches use (vl_stage_kernel)
     bool fuse_field = false;      // the loop's stage kernels solve for E themselves (vlasov_field_fuse.cuh)

@@ -28,7 +28,7 @@
 // resident warps, 128 registers each; more warps at fewer registers spill (n = 9 at 5 CTAs per SM: 1217
 // us).  Measured, Euler / combination stage, against the kernel that served the case before: FP32 n = 9 at
 // 64^3 714 / 865 us (paired-row TMA form 872 / 913), n = 7 at 24x31x33 32 / 40 (register-pencil kernel
-// 56 / 63), n = 4 at 32x64x64 27 / 32 (order-4 TMA kernel 40 / 48); FP64 n = 7 at 24x31x33 66 / 90
+// 56 / 63); FP64 n = 7 at 24x31x33 66 / 90
 // (generic kernel's cp.async form 119 / 147).
 #pragma once
 
