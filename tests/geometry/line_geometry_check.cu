@@ -1,0 +1,64 @@
+// Host check (no GPU) of the line-form stage kernel's shared-memory positions (vlasov_stage_line.cuh), for
+// every order, both precisions, every line of every thread (those past the last one too) and every number
+// of elements in a tile: a v line's values and its upwind trace lie in the tile buffer, in the line's own
+// row, and the trace is the neighbouring element's node or the one kept beside the tile.
+#include <cstdio>
+
+#include "vlasov_stage_line.cuh"
+
+static int failures = 0;
+
+static void expect(bool ok, const char *what, int n, int es, int r, int b, int nb) {
+    if (ok) return;
+    if (failures++ < 20) std::printf("FAIL n=%d element=%dB row=%d b=%d nb=%d: %s\n", n, es, r, b, nb, what);
+}
+
+template <int N, typename T>
+void check() {
+    using G = vl::LineGeom<N, T>;
+    const int es = (int)sizeof(T);
+    for (int tid = 0; tid < G::THREADS; ++tid)
+        for (int s = 0; s < G::L; ++s) {
+            // as in the kernel: line l of the thread
+            const int l = tid + s * G::THREADS;
+            const bool has = l < G::LINES;
+            const int r = has ? l % (N * N) : 0, b = has ? l / (N * N) : 1 << 20;
+            for (int nb = 1; nb <= G::EPT; ++nb) {
+                const int p = r * G::W + (b < nb ? b * N : 0);
+                expect(p >= 0 && p % G::VEC == 0 && p + N <= r * G::W + G::COLS && p + N <= G::BUF, "values", N, es, r,
+                       b, nb);
+                for (int pos = 0; pos < 2; ++pos) {
+                    const int to = vl::line_vtrace(r * G::W, b, nb, N, pos != 0);
+                    const bool beside = b >= nb || (pos ? b == 0 : b == nb - 1);
+                    expect(to == (beside ? -1 : pos ? p - 1 : p + N), "trace", N, es, r, b, nb);
+                    expect(to == -1 || (to >= r * G::W && to < r * G::W + nb * N && to < G::BUF), "trace in its row", N,
+                           es, r, b, nb);
+                }
+            }
+        }
+}
+
+template <typename T>
+void all() {
+    check<1, T>();
+    check<2, T>();
+    check<3, T>();
+    check<4, T>();
+    check<5, T>();
+    check<6, T>();
+    check<7, T>();
+    check<8, T>();
+    check<9, T>();
+    check<10, T>();
+}
+
+int main() {
+    all<double>();
+    all<float>();
+    if (failures) {
+        std::printf("%d failures\n", failures);
+        return 1;
+    }
+    std::printf("ALL OK\n");
+    return 0;
+}

@@ -161,6 +161,15 @@ __device__ __forceinline__ void line_contract(const LineTables<N, T> &tb, int z,
     }
 }
 
+// Position in the tile buffer of the upwind trace of element b's v line in the row that starts at `row`
+// (nb elements in the tile): the neighbouring element's node, or -1 for the trace kept beside the tile.
+// Lines past the last element (of a ragged tile, or of the CTA) take that one too: their value is dropped,
+// but the word before the first row is not the tile's.
+__host__ __device__ constexpr int line_vtrace(int row, int b, int nb, int n, bool pos) {
+    if (pos) return b > 0 && b < nb ? row + b * n - 1 : -1;
+    return b < nb - 1 ? row + (b + 1) * n : -1;
+}
+
 template <typename T>
 struct LinePair;
 template <>
@@ -358,11 +367,10 @@ stage_line_kernel(const StageArgs a, const __grid_constant__ LineTables<N, T> tb
         // v lines
 #pragma unroll
         for (int s = 0; s < L; ++s) {
-            const T *p = sIn + r[s] * W + (b[s] < nb ? b[s] * N : 0);
-            line_load<N, G::VEC>(p, x[s]);
+            line_load<N, G::VEC>(sIn + r[s] * W + (b[s] < nb ? b[s] * N : 0), x[s]);
             const bool pos = svl[s] >= (T)0;
-            const T *pn = pos ? (b[s] > 0 ? p - 1 : sH + r[s]) : (b[s] < nb - 1 ? p + N : sH + r[s]);
-            const T t = *pn;
+            const int to = line_vtrace(r[s] * W, b[s], nb, N, pos);
+            const T t = to >= 0 ? sIn[to] : sH[r[s]];
             tl[s] = pos ? t : x[s][0];
             tr[s] = pos ? x[s][N - 1] : t;
         }
