@@ -24,15 +24,17 @@ void check() {
             const bool has = l < G::LINES;
             const int r = has ? l % (N * N) : 0, b = has ? l / (N * N) : 1 << 20;
             for (int nb = 1; nb <= G::EPT; ++nb) {
-                const int p = r * G::W + (b < nb ? b * N : 0);
-                expect(p >= 0 && p % G::VEC == 0 && p + N <= r * G::W + G::COLS && p + N <= G::BUF, "values", N, es, r,
-                       b, nb);
+                const int bb = vl::line_elem(b, nb), p = r * G::W + bb * N;
+                expect(bb == (b < nb ? b : 0), "element", N, es, r, b, nb);
+                expect(p % G::VEC == 0 && p + N <= r * G::W + nb * N && p + N <= G::BUF, "values", N, es, r, b, nb);
                 for (int pos = 0; pos < 2; ++pos) {
-                    const int to = vl::line_vtrace(r * G::W, b, nb, N, pos != 0);
-                    const bool beside = b >= nb || (pos ? b == 0 : b == nb - 1);
-                    expect(to == (beside ? -1 : pos ? p - 1 : p + N), "trace", N, es, r, b, nb);
-                    expect(to == -1 || (to >= r * G::W && to < r * G::W + nb * N && to < G::BUF), "trace in its row", N,
-                           es, r, b, nb);
+                    if (vl::line_trace_beside(bb, nb, pos != 0)) continue;   // (r < N N: a row of the halo buffer)
+                    const int to = p + (pos ? -1 : N);
+                    expect(to >= r * G::W && to < r * G::W + nb * N, "trace in its row", N, es, r, b, nb);
+                }
+                if (b < nb) {
+                    expect(vl::line_trace_beside(bb, nb, true) == (b == 0), "left trace", N, es, r, b, nb);
+                    expect(vl::line_trace_beside(bb, nb, false) == (b == nb - 1), "right trace", N, es, r, b, nb);
                 }
             }
         }

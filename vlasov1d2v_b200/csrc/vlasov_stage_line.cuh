@@ -161,14 +161,11 @@ __device__ __forceinline__ void line_contract(const LineTables<N, T> &tb, int z,
     }
 }
 
-// Position in the tile buffer of the upwind trace of element b's v line in the row that starts at `row`
-// (nb elements in the tile): the neighbouring element's node, or -1 for the trace kept beside the tile.
-// Lines past the last element (of a ragged tile, or of the CTA) take that one too: their value is dropped,
-// but the word before the first row is not the tile's.
-__host__ __device__ constexpr int line_vtrace(int row, int b, int nb, int n, bool pos) {
-    if (pos) return b > 0 && b < nb ? row + b * n - 1 : -1;
-    return b < nb - 1 ? row + (b + 1) * n : -1;
-}
+// Element of the tile (nb elements) that v line b reads: its own, or the first for a line past the last one
+// (of a ragged tile, or of the CTA), whose values are dropped.
+__host__ __device__ constexpr int line_elem(int b, int nb) { return b < nb ? b : 0; }
+// Whether the upwind trace of the tile's element b is the one kept beside the tile, not a neighbour's node
+__host__ __device__ constexpr bool line_trace_beside(int b, int nb, bool pos) { return pos ? b == 0 : b == nb - 1; }
 
 template <typename T>
 struct LinePair;
@@ -367,10 +364,21 @@ stage_line_kernel(const StageArgs a, const __grid_constant__ LineTables<N, T> tb
         // v lines
 #pragma unroll
         for (int s = 0; s < L; ++s) {
-            line_load<N, G::VEC>(sIn + r[s] * W + (b[s] < nb ? b[s] * N : 0), x[s]);
+            const int bb = line_elem(b[s], nb);
+            const T *p = sIn + r[s] * W + bb * N;
+            line_load<N, G::VEC>(p, x[s]);
             const bool pos = svl[s] >= (T)0;
-            const int to = line_vtrace(r[s] * W, b[s], nb, N, pos);
-            const T t = to >= 0 ? sIn[to] : sH[r[s]];
+            const bool beside = line_trace_beside(bb, nb, pos);
+            const int to = pos ? -1 : N;
+            // FP64 selects the value (n = 7 at 24x31x33 64 us per Euler stage, 66 the other way), FP32 its
+            // address (n = 9 at 64^3 852 us per combination stage, 871 the other way)
+            T t;
+            if constexpr (sizeof(T) == 8) {
+                t = beside ? sH[r[s]] : p[to];
+            } else {
+                const T *pn = beside ? sH + r[s] : p + to;
+                t = *pn;
+            }
             tl[s] = pos ? t : x[s][0];
             tr[s] = pos ? x[s][N - 1] : t;
         }
