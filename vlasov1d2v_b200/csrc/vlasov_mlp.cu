@@ -427,8 +427,11 @@ __global__ void __launch_bounds__(GRAD_THREADS) mlp_grad_kernel(const __nv_bfloa
     if (8 * wp >= ncol) return;
     const int g = lane >> 2, t = lane & 3;
     float *gw = grad_w + w_off(l) + (size_t)(m0 + g) * N + n0 + 8 * wp + 2 * t;
-    *reinterpret_cast<float2 *>(gw) = make_float2(sum[0], sum[1]);
-    *reinterpret_cast<float2 *>(gw + (size_t)8 * N) = make_float2(sum[2], sum[3]);
+    // (single floats: grad_w may start on any float)
+    gw[0] = sum[0];
+    gw[1] = sum[1];
+    gw[(size_t)8 * N] = sum[2];
+    gw[(size_t)8 * N + 1] = sum[3];
 }
 
 // Adam on the FP32 master weights [in][out] and biases; refresh both bf16 layouts
