@@ -238,8 +238,8 @@ __host__ __device__ constexpr size_t dz_off(int l, size_t rows) { return (size_t
 // dZ of a hidden layer from the next layer's dZ (sD, K wide): W^T given as wb [HID][K]
 template <int K>
 __device__ __forceinline__ void backprop_hidden(const __nv_bfloat16 *sD, const __nv_bfloat16 *sW,
-                                                const float *__restrict__ Z, int n0, int row0, int nrows, int lane,
-                                                __nv_bfloat16 *__restrict__ dZ, __nv_bfloat16 *sNext) {
+                                                const float *__restrict__ Z, bool z8, int n0, int row0, int nrows,
+                                                int lane, __nv_bfloat16 *__restrict__ dZ, __nv_bfloat16 *sNext) {
     const int g = lane >> 2, t = lane & 3;
     float acc[ROWS / 16][2][4];
     layer_mma<K, 2>(sD, sW, n0, lane, acc);
@@ -253,7 +253,8 @@ __device__ __forceinline__ void backprop_hidden(const __nv_bfloat16 *sD, const _
                 const int r = 16 * mm + 8 * h + g, row = row0 + r;
                 float d0 = 0.f, d1 = 0.f;
                 if (row < nrows) {
-                    const float2 z = *reinterpret_cast<const float2 *>(Z + (size_t)row * HID + c);
+                    const float *pz = Z + (size_t)row * HID + c;
+                    const float2 z = z8 ? *reinterpret_cast<const float2 *>(pz) : make_float2(pz[0], pz[1]);
                     d0 = acc[mm][nn][2 * h] * gelu_d(z.x);
                     d1 = acc[mm][nn][2 * h + 1] * gelu_d(z.y);
                 }
@@ -287,13 +288,14 @@ __global__ void __launch_bounds__(32 * WARPS) mlp_backprop_kernel(const float *_
         *reinterpret_cast<uint32_t *>(dZ + dz_off(NL - 1, rows) + (size_t)row * OUT + c) = v;
     }
     const size_t hs = (size_t)nrows * HID;
+    const bool z8 = (reinterpret_cast<uintptr_t>(Z) & 7) == 0;   // (elsewhere single floats)
     weights_ready<1>();
-    backprop_hidden<OUT>(sD[0], sW[0], Z + 2 * hs, 2 * wp, row0, nrows, lane, dZ + dz_off(2, rows), sD[1]);
+    backprop_hidden<OUT>(sD[0], sW[0], Z + 2 * hs, z8, 2 * wp, row0, nrows, lane, dZ + dz_off(2, rows), sD[1]);
     weights_ready<0>();
     stage_weights<HID, HID>(sW[0], w.wb[1]);
-    backprop_hidden<HID>(sD[1], sW[1], Z + hs, 2 * wp, row0, nrows, lane, dZ + dz_off(1, rows), sD[0]);
+    backprop_hidden<HID>(sD[1], sW[1], Z + hs, z8, 2 * wp, row0, nrows, lane, dZ + dz_off(1, rows), sD[0]);
     weights_ready<0>();
-    backprop_hidden<HID>(sD[0], sW[0], Z, 2 * wp, row0, nrows, lane, dZ + dz_off(0, rows), sD[1]);
+    backprop_hidden<HID>(sD[0], sW[0], Z, z8, 2 * wp, row0, nrows, lane, dZ + dz_off(0, rows), sD[1]);
 }
 
 // Gradients.  CTA < GRAD_TILES: a 16 x 32 tile of one layer's gW (warp: 16 x 8) over all samples, which
