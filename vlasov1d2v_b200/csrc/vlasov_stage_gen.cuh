@@ -337,6 +337,10 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
     constexpr size_t S_IN = L::S_IN, S_FN = L::S_FN, S_XF = L::S_XF, S_UF = L::S_UF;
     constexpr size_t S_BG = L::S_BG, S_STAGE = L::S_STAGE;
     constexpr int FS = L::FS;        // second face side (elements)
+    // moment sums and v speeds formed in FP64 throughout.  FP32 n = 4 too, whose density and speeds were FP64
+    // in the kernel that served it before; here that costs 1% (64^3 48.9 / 53.7 against 48.4 / 53.4 us per
+    // Euler / combination stage, 32x62x62 96.4 against 96.3 us per step)
+    constexpr bool SUM64 = sizeof(T) == 8 || N == 4;
     __shared__ __align__(8) uint64_t gfull[2];   // TMA form: one mbarrier per stage
     __shared__ FuseShared<FUSE ? N : 1, FUSE ? NT : 32> sFuse;   // field solve in the prologue
 
@@ -680,16 +684,16 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
             const T uL0 = (sd0 >= 0.0) ? ufl.x : fu[0].x, uR0 = (sd0 >= 0.0) ? fu[N - 1].x : ufr.x;
             const T uL1 = (sd1 >= 0.0) ? ufl.y : fu[0].y, uR1 = (sd1 >= 0.0) ? fu[N - 1].y : ufr.y;
             T *pout = out + (size_t)Eg * sE_ + (size_t)i * sI + (size_t)Ag * sA + col;
-            float mf0 = 0.0f, mf1 = 0.0f;   // FP32: the tile's moment sums, added in FP64 after it
+            float mf0 = 0.0f, mf1 = 0.0f;   // !SUM64: the tile's moment sums, added in FP64 after it
             (void)mf0;
             (void)mf1;
 #pragma unroll
             for (int j = 0; j < N; ++j) {
-                // x and v speeds of row j (FP32: one conversion, the v speed formed in FP32)
+                // x and v speeds of row j (FP32 but n = 4: one conversion, the v speed formed in FP32)
                 T uxT, svT;
                 if constexpr (sizeof(T) == 4) {
                     uxT = (float)sUX[j];
-                    svT = kvf * uxT;
+                    svT = SUM64 ? (float)(accel * (nbfield * sUX[j])) : kvf * uxT;
                 } else {
                     const double uxd = sUX[j];
                     uxT = uxd;
@@ -797,7 +801,7 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
                         if (!pad1) gout[(size_t)(nx + 1) * sE_ + gb + 1] = fij.y;
                     }
                 }
-                if constexpr (sizeof(T) == 4) {
+                if constexpr (!SUM64) {
                     mf0 = fmaf((float)tb.wu[j], o.x, mf0);
                     mf1 = fmaf((float)tb.wu[j], o.y, mf1);
                 } else {
@@ -805,7 +809,7 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
                     mk1 = fma(tb.wu[j], (double)o.y, mk1);
                 }
             }
-            if constexpr (sizeof(T) == 4) {
+            if constexpr (!SUM64) {
                 mk0 += (double)mf0;
                 mk1 += (double)mf1;
             }
