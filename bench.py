@@ -329,6 +329,7 @@ def measure_precision(precision, steps, warmup, reps, dist, res=None, order=None
     torch.cuda.synchronize()
     g = capture_steps(run, steps)
 
+    launches, form = run.ctx.loop_launches(steps), run.ctx.stage_form
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     dist.barrier()
     torch.cuda.synchronize()
@@ -363,7 +364,7 @@ def measure_precision(precision, steps, warmup, reps, dist, res=None, order=None
             stage_ms.append(a.elapsed_time(b) / reps)
     finally:
         ctx.set_background(None)
-    # field solve (one 8-CTA cluster: Poisson solve from a density)
+    # standalone field solve (Poisson solve from a density)
     rho = torch.zeros((res[0], order), dtype=torch.float64, device=run.f.device)
     ctx.moment(run.f, rho)
     chg = (rho.mean() - rho).contiguous()
@@ -383,6 +384,7 @@ def measure_precision(precision, steps, warmup, reps, dist, res=None, order=None
     if not e2e:
         del g
         return {"precision": precision, "ms": ms, "steps": steps, "dof": n_dof, "bytes_per_dof_step": 8 * es,
+                "launches": launches, "stage_form": form,
                 "stage_ms": stage_ms, "field_ms": field_ms, "state_bytes": state_bytes,
                 "stage_bytes": [2 * es * n_dof, 3 * es * n_dof, 3 * es * n_dof]}
     # end to end through the public API with host buffers: pinned f0 -> device, K steps,
@@ -406,6 +408,7 @@ def measure_precision(precision, steps, warmup, reps, dist, res=None, order=None
     del g
     return {
         "precision": precision, "ms": ms, "steps": steps, "dof": n_dof, "bytes_per_dof_step": 8 * es,
+        "launches": launches, "stage_form": form,
         "stage_ms": stage_ms, "field_ms": field_ms, "e2e_ms": e2e_ms, "state_bytes": state_bytes,
         "stage_bytes": [2 * es * n_dof, 3 * es * n_dof, 3 * es * n_dof],
     }
@@ -553,6 +556,7 @@ def main():
                          "algorithmic_bytes_per_launch": per_launch,
                          "kernel": "stage_frag_kernel<double>" if prec == "fp64" else
                                    "stage_f32_kernel<kind, background split>",
+                         "stage_form": r["stage_form"], "loop_launches": r["launches"],
                          "algorithmic_bytes_per_dof_step": r["bytes_per_dof_step"],
                          "stage_ms": r["stage_ms"], "field_ms": r["field_ms"],
                          "step_effective_gbs": r["dof"] * r["bytes_per_dof_step"] / (ms_step * 1e-3) / 1e9,
@@ -581,8 +585,8 @@ def main():
                    "buffers, 3 buffers)", "parallelism": f"replicas x{world}"},
         "roofline": head["roofline"],
         "e2e": head["e2e"],
-        # per step: 3 stage kernels, which solve for the field; one moment and one close per call
-        "gpu_launches": 3 * args.steps + 2,
+        # of the timed call, by the route that its context takes on this device
+        "gpu_launches": results["fp64"]["launches"],
         "clocks": ck,
         "variants": {"fp32_mixed": {"value": out["fp32"]["value"], "dtype": "f32",
                                     "ms_per_step": out["fp32"]["ms_per_step"],

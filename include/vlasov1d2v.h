@@ -124,6 +124,14 @@ VL_API size_t vl_state_elems(const vl_ctx *ctx);
  * partials of the stage kernels                                                             */
 VL_API size_t vl_workspace_bytes(const vl_ctx *ctx);
 
+/* How the context's calls run, by its sizes, precision and the device: the form of its stage kernels
+ * ("fragment", "packed", "generic", "generic-tma", "generic-pairs", "line" or "pencil"; NULL for a null
+ * context), and the kernel launches of one vl_ssp_rk3_steps call of nsteps steps (-1 for a null context
+ * or nsteps < 0): three a step, a moment and a closing one where the stage kernels solve for the
+ * field, six a step and a moment elsewhere.                                                  */
+VL_API const char *vl_stage_form(const vl_ctx *ctx);
+VL_API int64_t vl_loop_launches(const vl_ctx *ctx, int32_t nsteps);
+
 /* ---- hot-path operators ------------------------------------------------------------------ */
 
 /* DGFlux.semi_discrete_rhs (main/fluxes.py:59-105): out[interior] = J_x F_x + J_u F_u + J_v F_v

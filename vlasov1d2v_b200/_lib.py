@@ -22,7 +22,8 @@ ABI_VERSION = 2
 # every symbol include/vlasov1d2v.h declares (checked by the CPU test suite)
 EXPORTED = (
     "vl_ctx_create", "vl_ctx_destroy", "vl_last_error", "vl_abi_version", "vl_state_elems",
-    "vl_workspace_bytes", "vl_rhs", "vl_rhs_weighted", "vl_moment", "vl_poisson", "vl_field_energy", "vl_adapt_dt",
+    "vl_workspace_bytes", "vl_stage_form", "vl_loop_launches", "vl_rhs", "vl_rhs_weighted", "vl_moment",
+    "vl_poisson", "vl_field_energy", "vl_adapt_dt",
     "vl_rk_stage", "vl_run_state_init", "vl_ssp_rk3_steps", "vl_sync_ghosts",
     "vl_sync_stage_ghosts", "vl_rhs_whole",
     "vl_ssp_rk3_steps_noalloc", "vl_initial_state", "vl_smooth_edges", "vl_interpolate",
@@ -93,6 +94,10 @@ def _declare(lib):
     lib.vl_state_elems.restype = ctypes.c_size_t
     lib.vl_workspace_bytes.argtypes = [vp]
     lib.vl_workspace_bytes.restype = ctypes.c_size_t
+    lib.vl_stage_form.argtypes = [vp]
+    lib.vl_stage_form.restype = ctypes.c_char_p
+    lib.vl_loop_launches.argtypes = [vp, ctypes.c_int32]
+    lib.vl_loop_launches.restype = ctypes.c_int64
     lib.vl_rhs.argtypes = [vp, vp, vp, vp, i, vp]
     lib.vl_rhs_weighted.argtypes = [vp, vp, vp, vp, i, _c_dbl_p, vp]
     lib.vl_moment.argtypes = [vp, vp, vp, vp]
@@ -141,7 +146,7 @@ def _declare(lib):
                                    i32, i32, i32, vp, vp]
     for name in EXPORTED:
         if name not in ("vl_last_error", "vl_abi_version", "vl_state_elems", "vl_workspace_bytes",
-                        "vl_ens_workspace_bytes", "vl_mlp_partial_floats"):
+                        "vl_stage_form", "vl_loop_launches", "vl_ens_workspace_bytes", "vl_mlp_partial_floats"):
             getattr(lib, name).restype = i
 
 

@@ -113,6 +113,15 @@ class NativeContext:
                                           device=self.device)
         return self._workspace
 
+    @property
+    def stage_form(self):
+        """The form of the context's stage kernels (``vl_stage_form``)."""
+        return self._lib.vl_stage_form(self.handle).decode()
+
+    def loop_launches(self, nsteps):
+        """Kernel launches of one ``ssp_rk3_steps`` call."""
+        return int(self._lib.vl_loop_launches(self.handle, int(nsteps)))
+
     def _check_state(self, t, name="state"):
         if t.dtype != self.dtype:
             raise TypeError(f"{name} dtype {t.dtype} != context precision {self.dtype}")

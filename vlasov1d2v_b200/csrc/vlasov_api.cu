@@ -1317,6 +1317,22 @@ size_t vl_workspace_bytes(const vl_ctx *c) {
     return c->fuse_field ? 2 * partials_bytes(c) + 2 * CONTROL_BYTES : partials_bytes(c);
 }
 
+const char *vl_stage_form(const vl_ctx *c) {
+    if (c == nullptr) return nullptr;
+    switch (c->stage_kernel) {
+        case VL_STAGE_FRAG: return c->cfg.precision == VL_FP64 ? "fragment" : "packed";
+        case VL_STAGE_GEN: return c->gen_tma ? "generic-tma" : c->gen_pair ? "generic-pairs" : "generic";
+        case VL_STAGE_LINE: return "line";
+        default: return "pencil";
+    }
+}
+
+int64_t vl_loop_launches(const vl_ctx *c, int32_t nsteps) {
+    if (c == nullptr || nsteps < 0) return -1;
+    if (nsteps == 0) return 1;   // the moment of f
+    return c->fuse_field ? 1 + 3 * (int64_t)nsteps + 1 : 1 + 6 * (int64_t)nsteps;
+}
+
 int vl_rhs(vl_ctx *c, const void *f, const double *E, void *out, int xhalo, void *stream) {
     if (!c || !f || !E || !out) return fail(VL_ERR_INVALID, "null argument");
     if (xhalo != VL_XHALO_GHOST && xhalo != VL_XHALO_PERIODIC) return fail(VL_ERR_INVALID, "xhalo");
