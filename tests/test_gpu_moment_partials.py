@@ -14,8 +14,8 @@ from test_gpu_line_kernel import _context, _inputs
 
 pytestmark = pytest.mark.gpu
 
-# FP64 sums: every FP64 kernel; in FP32 order 4 and the line-form kernel (orders 7, 9, odd rows)
-SUM64 = [(4, (2, 3, 5), "fp32"), (4, (3, 5, 16), "fp32"), (4, (2, 4, 33), "fp32"), (7, (2, 3, 5), "fp32"),
+# FP64 sums: every FP64 kernel; in FP32 orders 4 and 10 and the line-form kernel (orders 7, 9, odd rows)
+SUM64 = [(10, (32, 20, 20), "fp32"), (10, (2, 3, 4), "fp32"), (4, (2, 3, 5), "fp32"), (4, (3, 5, 16), "fp32"), (4, (2, 4, 33), "fp32"), (7, (2, 3, 5), "fp32"),
          (7, (3, 4, 6), "fp32"), (9, (2, 3, 4), "fp32"), (3, (2, 3, 4), "fp32"), (5, (2, 4, 7), "fp32"),
          (4, (2, 3, 5), "fp64"), (6, (3, 3, 8), "fp64"), (7, (2, 3, 5), "fp64"), (8, (2, 3, 6), "fp64"),
          (9, (2, 3, 4), "fp64")]

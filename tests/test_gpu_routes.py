@@ -72,6 +72,9 @@ def test_field_solved_in_the_stages(cuda, res, n, precision, split, monkeypatch)
     ((4, 6, 7), 7, "fp64", "line"), ((4, 6, 6), 9, "fp32", "line"), ((4, 6, 7), 7, "fp32", "line"),
     ((4, 6, 7), 5, "fp32", "line"), ((4, 6, 7), 4, "fp32", "generic-tma"), ((4, 6, 6), 6, "fp32", "generic-tma"),
     ((4, 6, 7), 6, "fp32", "generic-pairs"), ((4, 6, 6), 3, "fp32", "generic-tma"), ((2, 3, 5), 2, "fp32", "generic-pairs"),
+    # order 10: many tiles for each resident CTA or few
+    ((32, 40, 40), 10, "fp32", "generic-tma"), ((32, 40, 41), 10, "fp32", "generic-pairs"),
+    ((32, 20, 20), 10, "fp32", "generic-tma"), ((8, 12, 12), 10, "fp32", "line"), ((3, 4, 5), 10, "fp32", "line"),
     # an x slab of 4 GiB or more: past the line form's 32-bit offsets
     ((1, 1300, 1301), 9, "fp32", "pencil"), ((1, 1300, 1300), 9, "fp32", "generic-pairs"),
     ((1, 1300, 1301), 7, "fp64", "generic")])

@@ -1181,10 +1181,15 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
     //     combination stage against 119 / 147 in the generic kernel's cp.async form; on 16-byte rows the
     //     TMA form is faster: 83 / 89 against 88 / 121 us at 32^3)
     //   FP32, orders 2 to 6: the generic kernel's TMA forms where the rows allow them (n = 6 at 32x62x62
-    //     91 / 100 us against 97 / 116 in the line form, n = 4 26 / 28 against 27 / 31, n = 2 at 64x128x128 31 / 33 against 44 / 49)
-    //   FP32, other orders and rows: the line form (64^3, n = 9: 703 / 865 us against 870 / 912 in the
-    //     generic kernel's paired-row TMA form; n = 7 at 32x62x62 151 / 179 against 179 / 188 in its TMA
-    //     form, at 24x31x33 32 / 40 against 56 / 63 in the register-pencil kernel)
+    //     91 / 100 us against 97 / 116 in the line form, n = 5 63 / 68 against 66 / 72, n = 4 25 / 28 against
+    //     27 / 31, n = 3 17 / 18 against 22 / 24, n = 2 at 64x128x128 31 / 33 against 44 / 49)
+    //   FP32, order 10: the same on grids of more than 6 line-form tiles for each resident CTA (32x40x40
+    //     254 / 260 us against 275 / 301, 32x20x20 69 / 72 against 74 / 83: there the line form's spills, 110
+    //     to 170 bytes at this order alone, cost more than the generic form's one CTA per SM); the line form
+    //     on smaller ones (16^3 25 / 27 against 28 / 29, 8x12x12 8.8 / 9.5 against 10.7 / 10.9)
+    //   FP32, other orders and rows: the line form (64^3, n = 9: 723 / 852 us against 870 / 912 in the
+    //     generic kernel's paired-row TMA form; n = 7 at 32x62x62 155 / 180 against 179 / 188 in its TMA
+    //     form, at 24x31x33 33 / 41 against 56 / 63 in the register-pencil kernel)
     // The line form takes x slabs below 4 GiB (32-bit offsets); beyond, the generic and register-pencil
     // kernels serve its cases.  VLASOV1D2V_STAGE_KERNEL=frag|gen|pencil|line selects one of the forms
     // that apply, for comparisons; VLASOV1D2V_GEN_NO_TMA=1 keeps the generic kernel off its TMA forms.
@@ -1199,7 +1204,15 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
                             ((size_t)(cfg->nu + 2) * n) % 2 == 0 && !no_gen_tma && encode_fn() != nullptr;
     const bool line_ok = elems / (size_t)(cfg->nx + 2) * (cfg->precision == VL_FP64 ? 8 : 4) < ((size_t)1 << 32);
     const bool tma64 = ((size_t)(cfg->nv + 2) * n) % 2 == 0 && encode_fn() != nullptr && !no_gen_tma;
-    const bool tma_better = cfg->precision == VL_FP64 ? tma64 : (gen_tma32 || gen_pair32) && n >= 2 && n <= 6;
+    // (FP32 n = 10) more than 6 line-form tiles for each CTA that is resident
+    const bool many_tiles = [&] {
+        if (cfg->precision != VL_FP32 || n != 10) return false;
+        const int ept = vl::line_ept(n);
+        const int64_t tiles = (int64_t)cfg->nx * cfg->nu * ((cfg->nv + ept - 1) / ept);
+        return tiles > 6 * (int64_t)c->sm_count * vl::line_occupancy<float>(n, vl::KIND_COMBINE);
+    }();
+    const bool tma_better = cfg->precision == VL_FP64 ? tma64
+                                                      : (gen_tma32 || gen_pair32) && ((n >= 2 && n <= 6) || many_tiles);
     // the forms without the line kernel (they also say how the entry points want buffers aligned)
     const int general = cfg->precision == VL_FP64     ? VL_STAGE_GEN
                         : (gen_tma32 || gen_pair32)   ? VL_STAGE_GEN

@@ -337,10 +337,10 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
     constexpr size_t S_IN = L::S_IN, S_FN = L::S_FN, S_XF = L::S_XF, S_UF = L::S_UF;
     constexpr size_t S_BG = L::S_BG, S_STAGE = L::S_STAGE;
     constexpr int FS = L::FS;        // second face side (elements)
-    // moment sums and v speeds formed in FP64 throughout.  FP32 n = 4 too, whose density and speeds were FP64
-    // in the kernel that served it before; here that costs 1% (64^3 48.9 / 53.7 against 48.4 / 53.4 us per
-    // Euler / combination stage, 32x62x62 96.4 against 96.3 us per step)
-    constexpr bool SUM64 = sizeof(T) == 8 || N == 4;
+    // moment sums and v speeds formed in FP64 throughout.  FP32 n = 4 and 10 too, whose density and speeds are
+    // FP64 in the kernels that serve or served them elsewhere; here that costs 1% (n = 4 at 64^3 48.9 / 53.7
+    // against 48.4 / 53.4 us per Euler / combination stage)
+    constexpr bool SUM64 = sizeof(T) == 8 || N == 4 || N == 10;
     __shared__ __align__(8) uint64_t gfull[2];   // TMA form: one mbarrier per stage
     __shared__ FuseShared<FUSE ? N : 1, FUSE ? NT : 32> sFuse;   // field solve in the prologue
 
@@ -689,7 +689,7 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
             (void)mf1;
 #pragma unroll
             for (int j = 0; j < N; ++j) {
-                // x and v speeds of row j (FP32 but n = 4: one conversion, the v speed formed in FP32)
+                // x and v speeds of row j (without SUM64 one conversion, the v speed formed in FP32)
                 T uxT, svT;
                 if constexpr (sizeof(T) == 4) {
                     uxT = (float)sUX[j];
