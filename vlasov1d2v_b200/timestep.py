@@ -61,6 +61,9 @@ class NonFiniteError(FloatingPointError):
 _HIST_OFFSET = (_lib.RUN_STATE_BYTES + 127) // 128 * 128   # histories behind the loop state
 
 
+_BLOCK_COPY = 400 << 10   # bytes up to which one copy is cheaper than two and a gather (both 166 us a call)
+
+
 class _Run:
     """Device buffers of one (distribution, grids, physics) loop set-up."""
 
@@ -93,8 +96,14 @@ class _Run:
         """Copies of the field and the potential."""
         return _device.wrap(self.E.clone()), _device.wrap(self.phi.clone())
 
-    def read_batch(self):
-        """The loop state and the histories (energy, time, dt) on the host."""
+    def read_batch(self, limit=None):
+        """The loop state and the histories (energy, time, dt) on the host, of a batch of at most
+        ``limit`` steps."""
+        # one copy of the block, unless most of a long ring would travel unused: then the state, and
+        # the rows of the steps that it counts
+        if limit is not None and self.block.numel() > _BLOCK_COPY and 2 * limit < self.cap:
+            st = self.read_state()
+            return st, self.hist[:, :max(int(st.steps), 0)].cpu().numpy()
         raw = self.block.cpu().numpy()
         st = _lib.VlRunState.from_buffer_copy(raw[:_lib.RUN_STATE_BYTES])
         return st, raw[_HIST_OFFSET:].view(np.float64).reshape(3, self.cap)
@@ -308,7 +317,7 @@ class Stepper:
             run.upload_state(self._host_state(run, float("inf"), k))
             run.launch(k, False)
             fields = run.fields()   # enqueued before the host waits
-            st, h = run.read_batch()
+            st, h = run.read_batch(k)
             self.record(h, int(st.steps))
             if st.status != 0:
                 raise NonFiniteError("non-finite field or energy detected")
