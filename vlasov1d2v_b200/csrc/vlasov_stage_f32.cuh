@@ -64,6 +64,7 @@ stage_f32_kernel(const StageArgs a, const __grid_constant__ F32Tables tb, const 
     constexpr int N = G::N, P = G::P, W = G::W, PS = G::PS, WF = G::WF, PSF = G::PSF;
     constexpr int COLS = G::COLS, EPT = G::EPT;
     static_assert(G::THREADS == 128 && EPT == 4, "four warps of two x nodes each");
+    if (stage_skipped(a)) return;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(

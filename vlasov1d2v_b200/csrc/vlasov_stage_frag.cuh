@@ -129,6 +129,7 @@ stage_frag_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
     using V2 = typename Pair<T>::V;
     constexpr int N = G::N, P = G::P, W = G::W, PS = G::PS, WF = G::WF, PSF = G::PSF;
     constexpr int COLS = G::COLS, EPT = G::EPT, NT = G::THREADS;
+    if (stage_skipped(a)) return;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(

@@ -872,6 +872,7 @@ template <int N, typename T, int KT = -1, int BT = -1, bool FUSE = false>
 __global__ void __launch_bounds__(GenTmaGeom<N, T>::THREADS, GenTmaGeom<N, T>::MINB)
 stage_gen_tma_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
                      const __grid_constant__ GenMaps maps) {
+    if (stage_skipped(a)) return;
     extern __shared__ __align__(16) unsigned char gen_smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(gen_smem_raw) + 127) & ~(uintptr_t)127);
@@ -884,6 +885,7 @@ template <int N, typename T, int KT = -1, int BT = -1, bool FUSE = false>
 __global__ void __launch_bounds__(GenPairGeom<N, T>::THREADS, GenPairGeom<N, T>::MINB)
 stage_gen_pair_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
                       const __grid_constant__ GenMaps maps) {
+    if (stage_skipped(a)) return;
     extern __shared__ __align__(16) unsigned char gen_smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(gen_smem_raw) + 127) & ~(uintptr_t)127);

@@ -200,6 +200,7 @@ stage_line_kernel(const StageArgs a, const __grid_constant__ LineTables<N, T> tb
     constexpr int EPT = G::EPT, COLS = G::COLS, W = G::W, L = G::L, NN = N * N;
     constexpr uint32_t ES = sizeof(T);
     static_assert(BG == 0 || sizeof(T) == 4, "the background split is a form of FP32 states");
+    if (stage_skipped(a)) return;
 
     extern __shared__ __align__(128) unsigned char line_smem[];
     T *const sTile = reinterpret_cast<T *>(line_smem);   // two tile buffers
