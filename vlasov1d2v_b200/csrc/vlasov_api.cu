@@ -564,28 +564,9 @@ template <int N, typename T>
 int stage_occupancy_t(bool frag, bool gen, bool gtma, bool gpair) {
     int blocks = 0;
     if constexpr (sizeof(T) == 4) {
-        if (gen && gpair) {
-            using G = vl::GenPairGeom<N, T>;
-            const size_t smem = G::smem_bytes();
-            cudaFuncSetAttribute(vl::stage_gen_pair_kernel<N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
-            vl::gen_kinds_prepare<T>(N, true, smem);
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, vl::stage_gen_pair_kernel<N, T>, G::THREADS,
-                                                              smem) != cudaSuccess)
-                return 1;
-            return blocks > 0 ? blocks : 1;
-        }
+        if (gen && gpair) return vl::gen_kinds_prepare<T>(N, true, vl::GenPairGeom<N, T>::smem_bytes());
     }
-    if (gen && gtma) {
-        using G = vl::GenTmaGeom<N, T>;
-        const size_t smem = G::smem_bytes();
-        cudaFuncSetAttribute(vl::stage_gen_tma_kernel<N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        vl::gen_kinds_prepare<T>(N, false, smem);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, vl::stage_gen_tma_kernel<N, T>, G::THREADS,
-                                                          smem) != cudaSuccess)
-            return 1;
-        return blocks > 0 ? blocks : 1;
-    }
+    if (gen && gtma) return vl::gen_kinds_prepare<T>(N, false, vl::GenTmaGeom<N, T>::smem_bytes());
     if (gen) {
         using G = vl::GenGeom<N, T>;
         const size_t smem = G::smem_bytes();
@@ -617,12 +598,9 @@ int stage_occupancy_t(bool frag, bool gen, bool gtma, bool gpair) {
                                                                   G::THREADS, smem) != cudaSuccess)
                     return 1;
             } else {
-                cudaFuncSetAttribute(vl::stage_frag_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem);
-                cudaFuncSetAttribute(vl::stage_frag_kernel<T, true, vl::KIND_COMBINE>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, vl::stage_frag_kernel<T, true>,
-                                                                  G::THREADS, smem) != cudaSuccess)
+                constexpr auto k = &vl::stage_frag_kernel<T, true, vl::KIND_COMBINE>;
+                cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, G::THREADS, smem) != cudaSuccess)
                     return 1;
             }
             return blocks > 0 ? blocks : 1;
@@ -642,17 +620,17 @@ int stage_occupancy_t(bool frag, bool gen, bool gtma, bool gpair) {
 int frag_nofn_occupancy() {
     using G = vl::FragGeom<double, false>;
     const size_t smem = G::smem_bytes();
-    cudaFuncSetAttribute(vl::stage_frag_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-    cudaFuncSetAttribute(vl::stage_frag_kernel<double, false, vl::KIND_EULER>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(vl::stage_frag_kernel<double, false, vl::KIND_RHS>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, vl::stage_frag_kernel<double, false>, G::THREADS,
-                                                      smem) != cudaSuccess)
-        return 1;
-    return blocks > 0 ? blocks : 1;
+    int occ = 32;
+    auto one = [&](auto *k) {
+        int blocks = 0;
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, G::THREADS, smem) != cudaSuccess || blocks < 1)
+            blocks = 1;
+        occ = std::min(occ, blocks);
+    };
+    one(&vl::stage_frag_kernel<double, false, vl::KIND_EULER>);
+    one(&vl::stage_frag_kernel<double, false, vl::KIND_RHS>);
+    return occ;
 }
 
 template <typename T>

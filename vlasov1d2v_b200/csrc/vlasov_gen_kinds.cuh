@@ -53,24 +53,32 @@ cudaError_t launch_n(int kind, bool bg, dim3 grid, size_t smem, cudaStream_t s, 
     return launch_one<T, N, PAIR, KIND_RHS, 0>(grid, smem, s, a, tb, maps);
 }
 
+// shared-memory limits of every instantiation that launch_n launches, and the fewest CTAs of one that an SM
+// keeps resident
 template <typename T, int N, bool PAIR>
-void prepare_n(size_t smem) {
-    const int b = (int)smem;
-    cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_EULER, 0>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_COMBINE, 0>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_RHS, 0>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if constexpr (gen_fusable<T>(N, PAIR)) {
-        constexpr int B1 = sizeof(T) == 4 ? 1 : 0;
-        cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_EULER, 0, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-        cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_COMBINE, 0, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-        cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_EULER, B1, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-        cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_COMBINE, B1, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    }
-    if constexpr (sizeof(T) == 4) {
-        cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_EULER, 1>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-        cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_COMBINE, 1>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-        cudaFuncSetAttribute(kernel<T, N, PAIR, KIND_RHS, 1>(), cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    }
+int prepare_n(size_t smem) {
+    constexpr int THREADS = PAIR ? GenPairGeom<N, T>::THREADS : GenTmaGeom<N, T>::THREADS;
+    int occ = 32;
+    auto one = [&](auto *k) {
+        int blocks = 0;
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, THREADS, smem) != cudaSuccess || blocks < 1)
+            blocks = 1;
+        occ = blocks < occ ? blocks : occ;
+    };
+    auto kinds = [&](auto bc) {
+        constexpr int B = decltype(bc)::value;
+        one(kernel<T, N, PAIR, KIND_EULER, B>());
+        one(kernel<T, N, PAIR, KIND_COMBINE, B>());
+        one(kernel<T, N, PAIR, KIND_RHS, B>());
+        if constexpr (gen_fusable<T>(N, PAIR)) {
+            one(kernel<T, N, PAIR, KIND_EULER, B, true>());
+            one(kernel<T, N, PAIR, KIND_COMBINE, B, true>());
+        }
+    };
+    kinds(std::integral_constant<int, 0>{});
+    if constexpr (sizeof(T) == 4) kinds(std::integral_constant<int, 1>{});
+    return occ;
 }
 
 }  // namespace gk

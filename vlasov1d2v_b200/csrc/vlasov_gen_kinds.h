@@ -12,14 +12,15 @@
 namespace vl {
 
 // Launch stage kind `kind` of order n (1..10) with `bg` background-split tables; pair selects the
-// paired-row form (FP32 only).  grid / smem as for the run-time-kind instantiation.
+// paired-row form (FP32 only).  grid / smem: CTAs and dynamic shared memory.
 template <typename T>
 cudaError_t gen_kinds_launch(int n, bool pair, int kind, bool bg, dim3 grid, size_t smem, cudaStream_t s,
                              const StageArgs &a, const StageTables<T> &tb, const GenMaps &maps);
 
-// Allow `smem` bytes of dynamic shared memory for every instantiation of order n of the form.
+// Allow `smem` bytes of dynamic shared memory for every instantiation of order n of the form; returns the
+// resident CTAs per SM (the fewest of an instantiation).
 template <typename T>
-void gen_kinds_prepare(int n, bool pair, size_t smem);
+int gen_kinds_prepare(int n, bool pair, size_t smem);
 
 template <>
 cudaError_t gen_kinds_launch<double>(int n, bool pair, int kind, bool bg, dim3 grid, size_t smem, cudaStream_t s,
@@ -28,16 +29,16 @@ template <>
 cudaError_t gen_kinds_launch<float>(int n, bool pair, int kind, bool bg, dim3 grid, size_t smem, cudaStream_t s,
                                     const StageArgs &a, const StageTables<float> &tb, const GenMaps &maps);
 template <>
-void gen_kinds_prepare<double>(int n, bool pair, size_t smem);
+int gen_kinds_prepare<double>(int n, bool pair, size_t smem);
 template <>
-void gen_kinds_prepare<float>(int n, bool pair, size_t smem);
+int gen_kinds_prepare<float>(int n, bool pair, size_t smem);
 
 // the FP32 forms' instantiations, split over two translation units
 cudaError_t gen_kinds_launch_tma32(int n, int kind, bool bg, dim3 grid, size_t smem, cudaStream_t s,
                                    const StageArgs &a, const StageTables<float> &tb, const GenMaps &maps);
 cudaError_t gen_kinds_launch_pair32(int n, int kind, bool bg, dim3 grid, size_t smem, cudaStream_t s,
                                     const StageArgs &a, const StageTables<float> &tb, const GenMaps &maps);
-void gen_kinds_prepare_tma32(int n, size_t smem);
-void gen_kinds_prepare_pair32(int n, size_t smem);
+int gen_kinds_prepare_tma32(int n, size_t smem);
+int gen_kinds_prepare_pair32(int n, size_t smem);
 
 }  // namespace vl

@@ -21,19 +21,19 @@ cudaError_t gen_kinds_launch_tma32(int n, int kind, bool bg, dim3 grid, size_t s
     }
 }
 
-void gen_kinds_prepare_tma32(int n, size_t smem) {
+int gen_kinds_prepare_tma32(int n, size_t smem) {
     switch (n) {
-        case 1: gk::prepare_n<float, 1, false>(smem); break;
-        case 2: gk::prepare_n<float, 2, false>(smem); break;
-        case 3: gk::prepare_n<float, 3, false>(smem); break;
-        case 4: gk::prepare_n<float, 4, false>(smem); break;
-        case 5: gk::prepare_n<float, 5, false>(smem); break;
-        case 6: gk::prepare_n<float, 6, false>(smem); break;
-        case 7: gk::prepare_n<float, 7, false>(smem); break;
-        case 8: gk::prepare_n<float, 8, false>(smem); break;
-        case 9: gk::prepare_n<float, 9, false>(smem); break;
-        case 10: gk::prepare_n<float, 10, false>(smem); break;
-        default: break;
+        case 1: return gk::prepare_n<float, 1, false>(smem);
+        case 2: return gk::prepare_n<float, 2, false>(smem);
+        case 3: return gk::prepare_n<float, 3, false>(smem);
+        case 4: return gk::prepare_n<float, 4, false>(smem);
+        case 5: return gk::prepare_n<float, 5, false>(smem);
+        case 6: return gk::prepare_n<float, 6, false>(smem);
+        case 7: return gk::prepare_n<float, 7, false>(smem);
+        case 8: return gk::prepare_n<float, 8, false>(smem);
+        case 9: return gk::prepare_n<float, 9, false>(smem);
+        case 10: return gk::prepare_n<float, 10, false>(smem);
+        default: return 1;
     }
 }
 
@@ -45,11 +45,8 @@ cudaError_t gen_kinds_launch<float>(int n, bool pair, int kind, bool bg, dim3 gr
 }
 
 template <>
-void gen_kinds_prepare<float>(int n, bool pair, size_t smem) {
-    if (pair)
-        gen_kinds_prepare_pair32(n, smem);
-    else
-        gen_kinds_prepare_tma32(n, smem);
+int gen_kinds_prepare<float>(int n, bool pair, size_t smem) {
+    return pair ? gen_kinds_prepare_pair32(n, smem) : gen_kinds_prepare_tma32(n, smem);
 }
 
 }  // namespace vl

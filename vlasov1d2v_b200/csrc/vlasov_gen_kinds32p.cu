@@ -21,19 +21,19 @@ cudaError_t gen_kinds_launch_pair32(int n, int kind, bool bg, dim3 grid, size_t 
     }
 }
 
-void gen_kinds_prepare_pair32(int n, size_t smem) {
+int gen_kinds_prepare_pair32(int n, size_t smem) {
     switch (n) {
-        case 1: gk::prepare_n<float, 1, true>(smem); break;
-        case 2: gk::prepare_n<float, 2, true>(smem); break;
-        case 3: gk::prepare_n<float, 3, true>(smem); break;
-        case 4: gk::prepare_n<float, 4, true>(smem); break;
-        case 5: gk::prepare_n<float, 5, true>(smem); break;
-        case 6: gk::prepare_n<float, 6, true>(smem); break;
-        case 7: gk::prepare_n<float, 7, true>(smem); break;
-        case 8: gk::prepare_n<float, 8, true>(smem); break;
-        case 9: gk::prepare_n<float, 9, true>(smem); break;
-        case 10: gk::prepare_n<float, 10, true>(smem); break;
-        default: break;
+        case 1: return gk::prepare_n<float, 1, true>(smem);
+        case 2: return gk::prepare_n<float, 2, true>(smem);
+        case 3: return gk::prepare_n<float, 3, true>(smem);
+        case 4: return gk::prepare_n<float, 4, true>(smem);
+        case 5: return gk::prepare_n<float, 5, true>(smem);
+        case 6: return gk::prepare_n<float, 6, true>(smem);
+        case 7: return gk::prepare_n<float, 7, true>(smem);
+        case 8: return gk::prepare_n<float, 8, true>(smem);
+        case 9: return gk::prepare_n<float, 9, true>(smem);
+        case 10: return gk::prepare_n<float, 10, true>(smem);
+        default: return 1;
     }
 }
 

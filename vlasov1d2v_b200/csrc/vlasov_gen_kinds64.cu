@@ -24,20 +24,20 @@ cudaError_t gen_kinds_launch<double>(int n, bool pair, int kind, bool bg, dim3 g
 }
 
 template <>
-void gen_kinds_prepare<double>(int n, bool pair, size_t smem) {
-    if (pair) return;
+int gen_kinds_prepare<double>(int n, bool pair, size_t smem) {
+    if (pair) return 1;
     switch (n) {
-        case 1: gk::prepare_n<double, 1, false>(smem); break;
-        case 2: gk::prepare_n<double, 2, false>(smem); break;
-        case 3: gk::prepare_n<double, 3, false>(smem); break;
-        case 4: gk::prepare_n<double, 4, false>(smem); break;
-        case 5: gk::prepare_n<double, 5, false>(smem); break;
-        case 6: gk::prepare_n<double, 6, false>(smem); break;
-        case 7: gk::prepare_n<double, 7, false>(smem); break;
-        case 8: gk::prepare_n<double, 8, false>(smem); break;
-        case 9: gk::prepare_n<double, 9, false>(smem); break;
-        case 10: gk::prepare_n<double, 10, false>(smem); break;
-        default: break;
+        case 1: return gk::prepare_n<double, 1, false>(smem);
+        case 2: return gk::prepare_n<double, 2, false>(smem);
+        case 3: return gk::prepare_n<double, 3, false>(smem);
+        case 4: return gk::prepare_n<double, 4, false>(smem);
+        case 5: return gk::prepare_n<double, 5, false>(smem);
+        case 6: return gk::prepare_n<double, 6, false>(smem);
+        case 7: return gk::prepare_n<double, 7, false>(smem);
+        case 8: return gk::prepare_n<double, 8, false>(smem);
+        case 9: return gk::prepare_n<double, 9, false>(smem);
+        case 10: return gk::prepare_n<double, 10, false>(smem);
+        default: return 1;
     }
 }
 

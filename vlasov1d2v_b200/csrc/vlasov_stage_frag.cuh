@@ -119,9 +119,8 @@ struct Pair<float> {
     using V = float2;
 };
 
-// KT >= 0 fixes the stage kind at compile time (the instantiations the loop launches: no per-row
-// branches on it); -1 reads it from the arguments
-template <typename T, bool WFN, int KT = -1>
+// KT: the stage kind (no per-row branches on it)
+template <typename T, bool WFN, int KT>
 __global__ void __launch_bounds__(FragGeom<T, WFN>::THREADS, FragGeom<T, WFN>::MINB)
 stage_frag_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
                   const __grid_constant__ FragMaps maps) {
@@ -161,7 +160,7 @@ stage_frag_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
         El = e;
         Er = e + 2;
     }
-    const int kind = KT >= 0 ? KT : a.kind;   // compile-time in the loop's instantiations
+    constexpr int kind = KT;
     const bool with_fn = WFN && (kind == KIND_COMBINE);   // combination stages launch the WFN form
     const bool with_bg = G::BG && a.bg_rb != nullptr;
     const uint32_t tx_bytes = G::TX_IN + 4 * G::TX_FACE + (with_fn ? G::TX_FN : 0) + (with_bg ? 2 * G::TX_BG : 0) +

@@ -864,11 +864,10 @@ stage_gen_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb) {
     gen_stage_body<N, T, GenGeom<N, T>::EPT>(a, tb, tb.wv, blockIdx.y, blockIdx.x, gridDim.x, base);
 }
 
-// TMA form (16-byte-aligned state rows).  KT / BT >= 0 fix the stage kind and the background
-// split at compile time (the instantiations launched by the loop: no per-row branches on them);
-// -1 reads them from the arguments.  FUSE: the form that solves for E itself (vlasov_field_fuse.cuh), its
+// TMA form (16-byte-aligned state rows).  KT / BT: the stage kind and the background split (no per-row
+// branches on them).  FUSE: the form that solves for E itself (vlasov_field_fuse.cuh), its
 // own instantiation: in one kernel with the other its code costs the n = 9 form registers (64^3: 8%).
-template <int N, typename T, int KT = -1, int BT = -1, bool FUSE = false>
+template <int N, typename T, int KT, int BT, bool FUSE>
 __global__ void __launch_bounds__(GenTmaGeom<N, T>::THREADS, GenTmaGeom<N, T>::MINB)
 stage_gen_tma_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
                      const __grid_constant__ GenMaps maps) {
@@ -881,7 +880,7 @@ stage_gen_tma_kernel(const StageArgs a, const __grid_constant__ StageTables<T> t
 }
 
 // paired-row TMA form (FP32 rows of R = 2 mod 4 floats); KT / BT / FUSE as for the TMA form
-template <int N, typename T, int KT = -1, int BT = -1, bool FUSE = false>
+template <int N, typename T, int KT, int BT, bool FUSE>
 __global__ void __launch_bounds__(GenPairGeom<N, T>::THREADS, GenPairGeom<N, T>::MINB)
 stage_gen_pair_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
                       const __grid_constant__ GenMaps maps) {
