@@ -262,11 +262,7 @@ __device__ __forceinline__ void field_conv_body(const FieldArgs &a, int rank, in
             bad_any |= s_rank_bad[r];
         }
         const double energy = 0.5 * (etot.hi + etot.lo);
-        const double ab = a.accel * a.bfield;
-        const double s0 = fabs(a.umax);
-        const double s1 = fabs(maxE + fabs(ab * a.vmax));
-        const double s2 = fabs(a.accel * fabs(a.bfield * a.umax));
-        const double dtn = a.courant / (((s0 / a.dx) + (s1 / a.du)) + (s2 / a.dv));
+        const double dtn = adapted_dt(a, a.accel, a.bfield, maxE);
         const int64_t steps = st_steps + 1;
         const double time = st_time + dtn;
         st->dt_next = dtn;

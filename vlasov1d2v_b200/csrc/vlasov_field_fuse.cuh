@@ -42,11 +42,7 @@ __host__ __device__ constexpr size_t field_fuse_scratch(int nx, int n) { return 
 // its field), then the promotion to the next step
 __device__ __forceinline__ void fuse_close_step(const FieldFuse &f, vl_run_state &c, double energy, double max_e,
                                                 double accel, double bfield, bool keeper) {
-    const double ab = accel * bfield;
-    const double s0 = fabs(f.umax);
-    const double s1 = fabs(max_e + fabs(ab * f.vmax));
-    const double s2 = fabs(accel * fabs(bfield * f.umax));
-    const double dtn = f.courant / (((s0 / f.dx) + (s1 / f.du)) + (s2 / f.dv));
+    const double dtn = adapted_dt(f, accel, bfield, max_e);
     c.steps += 1;
     c.time += dtn;
     c.dt_next = dtn;

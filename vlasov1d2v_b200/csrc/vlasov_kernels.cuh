@@ -190,6 +190,17 @@ __device__ __forceinline__ dd shfl_down_dd(dd v, int off) {
     return r;
 }
 
+// Stepper.adapt_time_step of get_max_speeds (main/timestep.py:231-242): dt from the largest |a E|; `a` has
+// the set-up's umax, vmax, dx, du, dv and courant
+template <typename A>
+__device__ __forceinline__ double adapted_dt(const A &a, double accel, double bfield, double max_e) {
+    const double ab = accel * bfield;
+    const double s0 = fabs(a.umax);
+    const double s1 = fabs(max_e + fabs(ab * a.vmax));
+    const double s2 = fabs(accel * fabs(bfield * a.umax));
+    return a.courant / (((s0 / a.dx) + (s1 / a.du)) + (s2 / a.dv));
+}
+
 // block-wide double-double sum (all threads call); result valid in every thread
 __device__ __forceinline__ double block_sum_dd_rt(double v, double c, dd *scratch) {
     dd s = {v, c};
@@ -406,11 +417,7 @@ static __global__ void __launch_bounds__(SCALAR_THREADS) scalars_kernel(const Sc
             maxE = fmax(maxE, s_max[w]);
         }
         const double energy = 0.5 * (t.hi + t.lo);
-        const double ab = a.accel * a.bfield;
-        const double s0 = fabs(a.umax);
-        const double s1 = fabs(maxE + fabs(ab * a.vmax));
-        const double s2 = fabs(a.accel * fabs(a.bfield * a.umax));
-        const double dtn = a.courant / (((s0 / a.dx) + (s1 / a.du)) + (s2 / a.dv));
+        const double dtn = adapted_dt(a, a.accel, a.bfield, maxE);
         if (a.energy) *a.energy = energy;
         if (a.dt) *a.dt = dtn;
         if (a.init) {

@@ -631,8 +631,6 @@ int check(const char *where) {
     return VL_OK;
 }
 
-}  // namespace
-
 // beta^step as the FP32 product of its factors, one after another.  A training loop asks for one step after
 // the other, so a thread goes on from the product of its last call where beta is the same (a whole
 // product per call takes 25 us at step 16000); the value does not depend on it.
@@ -667,6 +665,8 @@ int dynamic_smem() {
     if (dev >= 0 && dev < 64) done[dev] = true;
     return VL_OK;
 }
+
+}  // namespace
 
 extern "C" {
 

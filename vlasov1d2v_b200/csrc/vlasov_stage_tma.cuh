@@ -4,11 +4,9 @@
 #pragma once
 
 #include <cuda.h>
+#include <cuda_runtime.h>
 
-#include <type_traits>
-
-#include "vlasov_kernels.cuh"
-#include "vlasov_stage.cuh"
+#include <cstdint>
 
 namespace vl {
 
