@@ -79,22 +79,23 @@ __device__ __forceinline__ void fuse_store(vl_run_state *s, const vl_run_state &
 
 // E at x element e into sh.E, dt into sh.dt; false when the step does not run (all threads of the grid
 // agree).  scratch: field_fuse_scratch bytes of shared memory.
-template <int N, int NT>
+// CONTROL: the step's first stage (FUSE_FIRST, FUSE_STEP), which keeps the books; the others are FUSE_FIELD.
+template <int N, int NT, bool CONTROL>
 __device__ __forceinline__ bool field_prologue(const StageArgs &a, int e, double *scratch, FuseShared<N, NT> &sh) {
     constexpr int NW = NT / 32, RS = N | 1, S = field_conv_stride(N);
     const FieldFuse &f = a.ff;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nx = a.nx, nn = nx * N;
-    const bool control = f.mode != FUSE_FIELD;
+    const bool close = CONTROL && f.mode == FUSE_STEP;
     vl_run_state c;
-    if (control && tid == 0) fuse_load(c, f.ctl_in);
+    if (CONTROL && tid == 0) fuse_load(c, f.ctl_in);
     // a step after the loop's end (the one that finds the end closes the last step, below): its record is the
     // last one's.  Read beside the field and tested after it, the word costs a running step nothing (32 steps
     // after the end at 20x27x29 n = 7 FP32 436 -> 200 us, 352 with separate solves)
-    const int ran = f.mode == FUSE_STEP ? f.ctl_in->active : 1;
+    const int ran = close ? f.ctl_in->active : 1;
     dd loc = {0.0, 0.0}, en = {0.0, 0.0};
     double mx = 0.0;
-    if (f.mode == FUSE_STEP) {
+    if (close) {
         for (int p = tid; p < nn; p += NT) {
             const double ev = f.E_prev[N + p];
             en = dd_gather(en, dd{f.xw[p % N] * (ev * ev), 0.0});
@@ -116,7 +117,7 @@ __device__ __forceinline__ bool field_prologue(const StageArgs &a, int e, double
         loc = dd_gather(loc, dd{rho, 0.0});
     }
     for (int off = 16; off > 0; off >>= 1) loc = dd_gather(loc, dd_shfl_xor(loc, off));
-    if (f.mode == FUSE_STEP) {
+    if (close) {
         for (int off = 16; off > 0; off >>= 1) {
             en = dd_gather(en, dd_shfl_xor(en, off));
             mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
@@ -124,8 +125,10 @@ __device__ __forceinline__ bool field_prologue(const StageArgs &a, int e, double
     }
     if (lane == 0) {
         sh.rho[warp] = loc;
-        sh.en[warp] = en;
-        sh.mx[warp] = mx;
+        if constexpr (CONTROL) {
+            sh.en[warp] = en;
+            sh.mx[warp] = mx;
+        }
     }
     __syncthreads();
     dd t = sh.rho[0];
@@ -133,9 +136,9 @@ __device__ __forceinline__ bool field_prologue(const StageArgs &a, int e, double
     for (int w = 1; w < NW; ++w) t = dd_gather(t, sh.rho[w]);
     const double mean = (t.hi + t.lo) / (double)nn;
     if (tid == 0) {
-        if (control) {
+        if constexpr (CONTROL) {
             const bool keeper = blockIdx.x == 0 && blockIdx.y == 0;
-            if (f.mode == FUSE_STEP && c.active) {
+            if (close && c.active) {
                 dd es = sh.en[0];
                 double m = sh.mx[0];
 #pragma unroll

@@ -148,7 +148,7 @@ stage_f32_kernel(const StageArgs a, const __grid_constant__ F32Tables tb, const 
     }
     if (KIND != KIND_RHS && a.ff.mode != FUSE_NONE) {
         // E at this x element while the first tile travels; the second stage is the scratch
-        if (!field_prologue<N, G::THREADS>(a, e, reinterpret_cast<double *>(stage_ptr(1)), sFuse)) {
+        if (!field_prologue<N, G::THREADS, KIND == KIND_EULER>(a, e, reinterpret_cast<double *>(stage_ptr(1)), sFuse)) {
             if (ntile_cta > 0) mbar_wait_bounded(&full[0], 0);   // no copy left in flight
             return;
         }

@@ -208,7 +208,7 @@ stage_frag_kernel(const StageArgs a, const __grid_constant__ StageTables<T> tb,
     }
     if (KT != KIND_RHS && a.ff.mode != FUSE_NONE) {
         // E at this x element while the first tile travels; the second stage is the scratch
-        if (!field_prologue<N, NT>(a, e, reinterpret_cast<double *>(stage_ptr(1)), sFuse)) {
+        if (!field_prologue<N, NT, KT == KIND_EULER>(a, e, reinterpret_cast<double *>(stage_ptr(1)), sFuse)) {
             if (ntile_cta > 0) mbar_wait_bounded(&full[0], 0);   // no copy left in flight
             return;
         }

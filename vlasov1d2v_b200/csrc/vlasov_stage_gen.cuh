@@ -544,7 +544,7 @@ __device__ __forceinline__ void gen_stage_body(const StageArgs &a, const TB &tb,
             // E at this x element while the first tile travels; the second stage is the scratch, cleared
             // again for its pad columns
             unsigned char *sc = stage_ptr(1);
-            if (!field_prologue<N, NT>(a, e, reinterpret_cast<double *>(sc), sFuse)) {
+            if (!field_prologue<N, NT, KT == KIND_EULER>(a, e, reinterpret_cast<double *>(sc), sFuse)) {
                 if (ntile > 0) mbar_wait_bounded(&gfull[0], 0);   // no copy left in flight
                 return;
             }

@@ -297,7 +297,7 @@ stage_line_kernel(const StageArgs a, const __grid_constant__ LineTables<N, T> tb
     if (au < nu) load_tile(au, bt);
     if (KIND != KIND_RHS && a.ff.mode != FUSE_NONE) {
         // E at this x element while the first tile travels; the tile buffers are the scratch
-        if (!field_prologue<N, G::THREADS>(a, e, reinterpret_cast<double *>(line_smem), sFuse)) return;
+        if (!field_prologue<N, G::THREADS, KIND == KIND_EULER>(a, e, reinterpret_cast<double *>(line_smem), sFuse)) return;
     }
     const double accel = a.accel, bfield = a.bfield;
     const double dtd = (KIND == KIND_RHS) ? 0.0 : a.ff.mode != FUSE_NONE ? sFuse.dt : *a.dt;
