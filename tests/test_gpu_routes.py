@@ -51,8 +51,14 @@ def test_launches_are_those_of_a_captured_call(cuda, res, n, precision, form, mo
     assert run.ctx.loop_launches(0) == 1
 
 
-# order 10 has no stepper set-up of its own: its context's route alone
-@pytest.mark.parametrize("res,n,precision,split", CASES + [((3, 4, 4), 10, "fp64", False), ((3, 4, 5), 10, "fp64", False),
+# the grids of test_gpu_launch_overlap.py, whose kernels are launched as the one before ends only on this route
+OVERLAP = [((1, 1, 1), 6, "fp64", False), ((16, 16, 16), 8, "fp64", False), ((16, 16, 16), 8, "fp32", False),
+           ((8, 9, 9), 7, "fp32", False), ((5, 7, 9), 5, "fp64", False), ((16, 20, 20), 6, "fp64", False),
+           ((12, 24, 24), 5, "fp32", False), ((4, 40, 40), 9, "fp64", False)]
+
+
+# (order 10 has no stepper of its own: its context's route alone)
+@pytest.mark.parametrize("res,n,precision,split", CASES + OVERLAP + [((3, 4, 4), 10, "fp64", False), ((3, 4, 5), 10, "fp64", False),
                                                            ((3, 4, 4), 10, "fp32", False)])
 def test_field_solved_in_the_stages(cuda, res, n, precision, split, monkeypatch):
     """The small grids of the loop tests take the loop with the solve inside (all but FP32 order 2, whose
@@ -72,6 +78,10 @@ def test_field_solved_in_the_stages(cuda, res, n, precision, split, monkeypatch)
     ((4, 6, 7), 7, "fp64", "line"), ((4, 6, 6), 9, "fp32", "line"), ((4, 6, 7), 7, "fp32", "line"),
     ((4, 6, 7), 5, "fp32", "line"), ((4, 6, 7), 4, "fp32", "generic-tma"), ((4, 6, 6), 6, "fp32", "generic-tma"),
     ((4, 6, 7), 6, "fp32", "generic-pairs"), ((4, 6, 6), 3, "fp32", "generic-tma"), ((2, 3, 5), 2, "fp32", "generic-pairs"),
+    # the grid of the line kernel's comparison with the generic forms
+    ((2, 3, 5), 3, "fp64", "line"), ((2, 3, 5), 5, "fp64", "line"), ((2, 3, 5), 7, "fp64", "line"),
+    ((2, 3, 5), 9, "fp64", "line"), ((2, 3, 5), 3, "fp32", "line"), ((2, 3, 5), 5, "fp32", "line"),
+    ((2, 3, 5), 7, "fp32", "line"), ((2, 3, 5), 9, "fp32", "line"),
     # order 10: many tiles for each resident CTA or few
     ((32, 40, 40), 10, "fp32", "generic-tma"), ((32, 40, 41), 10, "fp32", "generic-pairs"),
     ((32, 20, 20), 10, "fp32", "generic-tma"), ((8, 12, 12), 10, "fp32", "line"), ((3, 4, 5), 10, "fp32", "line"),
