@@ -1155,19 +1155,19 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
     // Stage kernel (fastest measured per order and precision):
     //   n = 8: the fragment kernel (FP64), the packed-FP32 kernel (FP32)
     //   FP64, other orders: the generic kernel's TMA form where the rows are 16-byte multiples ((nv+2) n
-    //     even); the line form elsewhere (n = 7 at 24x31x33, odd rows: 66 / 90 us per Euler /
-    //     combination stage against 119 / 147 in the generic kernel's cp.async form; on 16-byte rows the
-    //     TMA form is faster: 83 / 89 against 88 / 121 us at 32^3)
-    //   FP32, orders 2 to 6: the generic kernel's TMA forms where the rows allow them (n = 6 at 32x62x62
-    //     91 / 100 us against 97 / 116 in the line form, n = 5 63 / 68 against 66 / 72, n = 4 25 / 28 against
-    //     27 / 31, n = 3 17 / 18 against 22 / 24, n = 2 at 64x128x128 31 / 33 against 44 / 49)
+    //     even); the line form elsewhere (n = 7 at 24x31x33, odd rows: 64 / 90 us per Euler /
+    //     combination stage against 117 / 144 in the generic kernel's cp.async form; on 16-byte rows the
+    //     TMA form is faster: 79 / 88 against 87 / 123 us at 32^3)
+    //   FP32, orders 2 to 6: the generic kernel's TMA forms where the rows allow them (32x62x62, us against
+    //     the line form: n = 2 7.0 / 7.1 to 8.3 / 8.7, n = 3 17 / 18 to 22 / 25, n = 4 25 / 28 to 27 / 31,
+    //     n = 5 63 / 68 to 64 / 71, n = 6 91 / 99 to 98 / 113)
     //   FP32, order 10: the same on grids of more than 6 line-form tiles for each resident CTA (32x40x40
     //     254 / 260 us against 275 / 301, 32x20x20 69 / 72 against 74 / 83: there the line form's spills, 110
     //     to 170 bytes at this order alone, cost more than the generic form's one CTA per SM); the line form
     //     on smaller ones (16^3 25 / 27 against 28 / 29, 8x12x12 8.8 / 9.5 against 10.7 / 10.9)
-    //   FP32, other orders and rows: the line form (64^3, n = 9: 723 / 852 us against 870 / 912 in the
-    //     generic kernel's paired-row TMA form; n = 7 at 32x62x62 155 / 180 against 179 / 188 in its TMA
-    //     form, at 24x31x33 33 / 41 against 56 / 63 in the register-pencil kernel)
+    //   FP32, other orders and rows: the line form (64^3, n = 9: 717 / 854 us against 872 / 914 in the
+    //     generic kernel's paired-row TMA form; n = 7 at 32x62x62 155 / 179 against 179 / 187 in its TMA
+    //     form, at 24x31x33 33 / 40 against 55 / 63 in the register-pencil kernel)
     // The line form takes x slabs below 4 GiB (32-bit offsets); beyond, the generic and register-pencil
     // kernels serve its cases.  VLASOV1D2V_STAGE_KERNEL=frag|gen|pencil|line selects one of the forms
     // that apply, for comparisons; VLASOV1D2V_GEN_NO_TMA=1 keeps the generic kernel off its TMA forms.
@@ -1256,8 +1256,8 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
         const char *env = getenv("VLASOV1D2V_FIELD");
         // (a CTA that starts in a later wave repeats the solve where the SMs would have stages to run: on
         // grids of more than one wave separate solves are as fast or faster, n = 8 at 64x32x32 501 against
-        // 509 us per step; in one wave the fused form is, 57 against 67 us at 16x20x20 n = 6, 579 against
-        // 594 at 32x50x50 n = 8)
+        // 509 us per step; in one wave the fused form is, 52.5 against 64 us at 16x20x20 n = 6, 575 against
+        // 585 at 32x50x50 n = 8)
         const bool one_wave = c->stage_grid_g * cfg->nx <= c->stage_slots && c->stage_grid_g1 * cfg->nx <= slots1;
         c->fuse_field = c->d_ke != nullptr && one_wave && room >= vl::field_fuse_scratch(cfg->nx, n) &&
                         !(env && std::string(env) == "solve");

@@ -14,10 +14,11 @@
 // date at the end of a batch.
 //
 // Bound by latency: partials, two block reductions, the dot products, 2 to 4 us where a separate solve and
-// the gap before it cost 6 to 8.  Per step, separate solves against this: 66 -> 56 us at 16x20x20 n = 6,
-// 69 -> 57 at 16^3 n = 8, 36 -> 27 at 8x12x12 n = 4, 593 -> 579 at 32x50x50 n = 8 (FP64).  Not in FP32 at
-// n = 2, whose small CTAs sum the partials slowly (24x30x30 45 -> 52 us); a called instead of an inlined
-// prologue costs the n = 8 stage 7 us of 160 in stack frames.
+// the gap before it cost 6 to 8.  Per step, separate solves against this (whose stages are also launched as
+// the one before ends): 64 -> 52.5 us at 16x20x20 n = 6, 68 -> 53.5 at 16^3 n = 8, 32 -> 22.6 at 8x12x12 n = 4,
+// 585 -> 575 at 32x50x50 n = 8 (FP64).  Not in FP32 at n = 2, whose small CTAs sum the partials slowly
+// (24x30x30 45 -> 52 us); a called instead of an inlined prologue costs the n = 8 stage 7 us of 160 in stack
+// frames.
 #pragma once
 
 #include "vlasov_field_conv.cuh"

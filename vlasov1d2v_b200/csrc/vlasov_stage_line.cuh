@@ -10,13 +10,13 @@
 // output per line), and every coefficient is a kernel-parameter operand that serves L lines: an FP64
 // FMA with a parameter operand runs at half rate when each serves one line (31.6 against 61 FMA per
 // clock and SM with two, measured), and in FP32 two lines share the addresses and tile arithmetic
-// (n = 9 at 64^3: Euler stage 703 against 838 us with one).
+// (n = 9 at 64^3: 16% less per Euler stage than with one).
 //
 // Per tile:
 //   barrier -> v lines (terms to RV), x lines (terms to RX), meanwhile the next tile's nodes travel
 //   from global memory into registers (lanes along the contiguous v columns) and then into the other
 //   tile buffer, and f^n by cp.async into its own (each thread reads what it copied itself; held in
-//   registers, f^n made the combination stage spill: 936 against 865 us) -> barrier -> u lines, RK
+//   registers, f^n made the combination stage spill: 8% slower at 64^3 n = 9) -> barrier -> u lines, RK
 //   combination, store (lanes along the columns)
 // Plain loads take any row alignment: one form serves every order and grid in both precisions (the
 // tensor-copy forms need rows, or pairs of rows, of 16-byte multiples).
@@ -24,12 +24,13 @@
 // Row strides in shared memory are an odd number of vectors, so the v phase's loads (lanes along
 // rows) fall in distinct banks; the x and u phases' lanes run along the columns.
 //
-// What bounds it: instruction issue (FP32 n = 9: about 75 instructions per value, 40 of them FMAs) at 16
-// resident warps, 128 registers each; more warps at fewer registers spill (n = 9 at 5 CTAs per SM: 1217
-// us).  Measured, Euler / combination stage, against the kernel that served the case before: FP32 n = 9 at
-// 64^3 714 / 865 us (paired-row TMA form 872 / 913), n = 7 at 24x31x33 32 / 40 (register-pencil kernel
-// 56 / 63); FP64 n = 7 at 24x31x33 66 / 90
-// (generic kernel's cp.async form 119 / 147).
+// What bounds it: FP32 instruction issue and the next tile's loads (n = 9: 88 / 97 instructions per value in
+// an Euler / combination stage, 58% issue active) at 16 resident warps, 128 registers each; more warps at
+// fewer registers spill (n = 9 at 5 CTAs per SM 40% slower).  FP64 the latency of loads and shared-memory
+// results at 12 warps.  Measured, Euler / combination stage in us, against the form that would serve the case
+// otherwise: FP32 n = 9 at 64^3 717 / 854 (paired-row TMA form 872 / 914), with the background split
+// 782 / 899 (931 / 994), n = 7 at 24x31x33 33 / 40 (register-pencil kernel 55 / 63); FP64 n = 7 at 24x31x33
+// 64 / 90 (generic kernel's cp.async form 117 / 144).
 #pragma once
 
 #include <cuda_runtime.h>
