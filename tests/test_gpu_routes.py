@@ -82,7 +82,8 @@ def test_field_solved_in_the_stages(cuda, res, n, precision, split, monkeypatch)
     ((2, 3, 5), 3, "fp64", "line"), ((2, 3, 5), 5, "fp64", "line"), ((2, 3, 5), 7, "fp64", "line"),
     ((2, 3, 5), 9, "fp64", "line"), ((2, 3, 5), 3, "fp32", "line"), ((2, 3, 5), 5, "fp32", "line"),
     ((2, 3, 5), 7, "fp32", "line"), ((2, 3, 5), 9, "fp32", "line"),
-    # order 10: many tiles for each resident CTA or few
+    # order 10: by the tiles of a resident CTA (a grid of few whose last line-form turn is nearly empty, too)
+    ((8, 17, 19), 10, "fp32", "generic-pairs"), ((16, 16, 16), 10, "fp32", "line"), ((8, 20, 21), 10, "fp32", "line"),
     ((32, 40, 40), 10, "fp32", "generic-tma"), ((32, 40, 41), 10, "fp32", "generic-pairs"),
     ((32, 20, 20), 10, "fp32", "generic-tma"), ((8, 12, 12), 10, "fp32", "line"), ((3, 4, 5), 10, "fp32", "line"),
     # an x slab of 4 GiB or more: past the line form's 32-bit offsets

@@ -1161,10 +1161,11 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
     //   FP32, orders 2 to 6: the generic kernel's TMA forms where the rows allow them (32x62x62, us against
     //     the line form: n = 2 7.0 / 7.1 to 8.3 / 8.7, n = 3 17 / 18 to 22 / 25, n = 4 25 / 28 to 27 / 31,
     //     n = 5 63 / 68 to 64 / 71, n = 6 91 / 99 to 98 / 113)
-    //   FP32, order 10: the same on grids of more than 6 line-form tiles for each resident CTA (32x40x40
-    //     254 / 260 us against 275 / 301, 32x20x20 69 / 72 against 74 / 83: there the line form's spills, 110
-    //     to 170 bytes at this order alone, cost more than the generic form's one CTA per SM); the line form
-    //     on smaller ones (16^3 25 / 27 against 28 / 29, 8x12x12 8.8 / 9.5 against 10.7 / 10.9)
+    //   FP32, order 10: the same where it is done first (32x40x40 254 / 260 us against 275 / 301, 32x20x20
+    //     69 / 72 against 74 / 83, 8x17x19 18.5 / 19.0 against 19.6 / 21.2: the line form's spills, 110 to 170
+    //     bytes at this order alone, cost more than the generic form's one CTA per SM); elsewhere, on small
+    //     grids and on 64 x elements of few tiles, the line form (16^3 25 / 27 against 28 / 29, 64x16x17
+    //     105 / 111 against 121 / 128)
     //   FP32, other orders and rows: the line form (64^3, n = 9: 717 / 854 us against 872 / 914 in the
     //     generic kernel's paired-row TMA form; n = 7 at 32x62x62 155 / 179 against 179 / 187 in its TMA
     //     form, at 24x31x33 33 / 40 against 55 / 63 in the register-pencil kernel)
@@ -1182,15 +1183,21 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
                             ((size_t)(cfg->nu + 2) * n) % 2 == 0 && !no_gen_tma && encode_fn() != nullptr;
     const bool line_ok = elems / (size_t)(cfg->nx + 2) * (cfg->precision == VL_FP64 ? 8 : 4) < ((size_t)1 << 32);
     const bool tma64 = ((size_t)(cfg->nv + 2) * n) % 2 == 0 && encode_fn() != nullptr && !no_gen_tma;
-    // (FP32 n = 10) more than 6 line-form tiles for each CTA that is resident
-    const bool many_tiles = [&] {
-        if (cfg->precision != VL_FP32 || n != 10) return false;
-        const int ept = vl::line_ept(n);
-        const int64_t tiles = (int64_t)cfg->nx * cfg->nu * ((cfg->nv + ept - 1) / ept);
-        return tiles > 6 * (int64_t)c->sm_count * vl::line_occupancy<float>(n, vl::KIND_COMBINE);
+    // (FP32 n = 10) whether the generic form is done first: 1.9 of its tiles take as long as a line-form tile
+    // where a resident CTA has several, and its grid may fill the device better or worse
+    const bool gen_first = [&] {
+        if (cfg->precision != VL_FP32 || n != 10 || !(gen_tma32 || gen_pair32)) return false;
+        auto turns = [&](int ept, int occ) {   // tiles of a resident CTA one after another
+            const int t = cfg->nu * ((cfg->nv + ept - 1) / ept), slots = c->sm_count * occ;
+            const int g = wave_grid(t, cfg->nx, slots);
+            return ((g * cfg->nx + slots - 1) / slots) * ((t + g - 1) / g);
+        };
+        const int line = turns(vl::line_ept(n), vl::line_occupancy<float>(n, vl::KIND_COMBINE));
+        const int gen = turns(gen_ept<float>(n), stage_occupancy<float>(n, false, true, gen_tma32, gen_pair32));
+        return line > 1 && 10 * gen < 19 * line;
     }();
     const bool tma_better = cfg->precision == VL_FP64 ? tma64
-                                                      : (gen_tma32 || gen_pair32) && ((n >= 2 && n <= 6) || many_tiles);
+                                                      : (gen_tma32 || gen_pair32) && ((n >= 2 && n <= 6) || gen_first);
     // the forms without the line kernel (they also say how the entry points want buffers aligned)
     const int general = cfg->precision == VL_FP64     ? VL_STAGE_GEN
                         : (gen_tma32 || gen_pair32)   ? VL_STAGE_GEN
