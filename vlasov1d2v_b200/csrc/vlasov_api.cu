@@ -555,7 +555,12 @@ int launch_line(vl_ctx *c, const vl::StageArgs &a0, cudaStream_t s) {
 }
 
 int stage(vl_ctx *c, const vl::StageArgs &a, cudaStream_t s) {
-    if (c->stage_kernel == VL_STAGE_LINE) return launch_line(c, a, s);
+    if (c->stage_kernel == VL_STAGE_LINE) {
+        if (a.kind != vl::KIND_RHS || c->rhs_pencil_g == 0) return launch_line(c, a, s);
+        vl::StageArgs b = a;
+        b.grid_g = c->rhs_pencil_g;
+        return launch_stage<float>(c, b, s);
+    }
     return c->cfg.precision == VL_FP64 ? launch_stage<double>(c, a, s)
                                        : launch_stage<float>(c, a, s);
 }
@@ -1209,9 +1214,11 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
                       : tma_better                                     ? VL_STAGE_GEN
                       : line_ok                                        ? VL_STAGE_LINE
                                                                        : general;
+    bool forced = false;
     {
         const char *env = getenv("VLASOV1D2V_STAGE_KERNEL");
         if (env) {
+            forced = env[0] != '\0';
             const std::string k(env);
             if (k == "gen") c->stage_kernel = VL_STAGE_GEN;
             else if (k == "pencil") c->stage_kernel = VL_STAGE_PENCIL;
@@ -1249,6 +1256,15 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
         const int lo1 = std::min(occ_of(vl::KIND_EULER), occ_of(vl::KIND_RHS));
         c->stage_grid_g1 = line_grid(lo1);
         slots1 = c->sm_count * lo1;
+        // FP32 n = 3: the line form's tiles of 28 v elements leave much of a row's last tile empty where nv is
+        // just above a multiple.  A right-hand side then runs on the register-pencil kernel (tiles of 10):
+        // 64x57x29 16.0 us against 24.4, 32x61x57 16.3 against 17.9; 32x61x85 24.4 either way, 16x31x25 4.5
+        // against 3.7.  The loop's stages stay, for the field solve inside them (64x72x57 168 us per step
+        // against 184 on the register-pencil kernel).
+        if (!forced && !d && n == 3 && general == VL_STAGE_PENCIL && 4 * cfg->nv < 3 * ept * ((cfg->nv + ept - 1) / ept)) {
+            const int pt = 32 / n, ptiles = cfg->nu * ((cfg->nv + pt - 1) / pt);
+            c->rhs_pencil_g = wave_grid(ptiles, cfg->nx, c->sm_count * stage_occupancy<float>(n, false, false, false, false));
+        }
     }
     {
         // the field solve inside the stage kernels: tables, a kernel that has the prologue, room for the

@@ -23,6 +23,8 @@ struct vl_ctx {
                         // f^n tile that fits more CTAs per SM; elsewhere = stage_grid_g)
     int stage_slots;    // resident CTAs of the combination stage's kernel on the device
     int stage_tiles;    // tiles per x element of the stage kernel
+    int rhs_pencil_g = 0;   // > 0: a right-hand side alone runs on the register-pencil kernel, with this many
+                            // CTAs per x element, where the stages run on the line form
     int moment_grid_g;  // CTAs per x element of the standalone moment kernel
     double up[vl::NMAX * vl::NMAX];
     double xi[vl::NMAX * 2];
