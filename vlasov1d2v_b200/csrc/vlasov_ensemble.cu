@@ -262,6 +262,7 @@ struct vl_ens {
     bool by_order = false;
     std::vector<Group> groups;
     std::vector<char> native;   // by order: member i launched through its own context
+    std::vector<char> own;      // and on that context's own grids
     // the launches of one by-order stage (one per ordinary group, one per member of a native
     // group) run concurrently: launch q on lane q mod LANES (lane 0 the caller's stream, lane k > 0
     // side[k - 1]), the side streams forked from and joined back into the caller's stream by
@@ -373,7 +374,7 @@ int native_stage(vl_ens *E, int i, int st, cudaStream_t s) {
     a.err = m.a.err;
     a.partials = m.a.partials;
     a.xhalo = m.a.xhalo;
-    a.grid_g = E->G[i];
+    a.grid_g = E->own[i] ? 0 : E->G[i];
     vl::ens_stage_args(a, m, st);
     return vl_internal_stage(c, a, s);
 }
@@ -530,6 +531,8 @@ int commit(vl_ens *E) {
             }
         E->members[i].G = G;
         for (int k = 0; k < 3; ++k) E->field[k][i].G = G;
+        // (on its context's own grids: the solve after the Euler stage reads that stage's partials)
+        if (E->own[i]) E->field[1][i].G = c->stage_grid_g1;
         E->field_smem = std::max(E->field_smem, E->conv ? vl::field_conv_smem(c->cfg.nx, c->cfg.n, true)
                                                         : vl::field_solve_smem(c->cfg.n, c->cfg.n_modes));
     }
@@ -599,6 +602,7 @@ VL_API int vl_ens_create(vl_ctx *const *ctxs, int32_t count, vl_ens **out) {
     for (int k = 0; k < 3; ++k) E->field[k].resize(count);
     E->bound.assign(count, 0);
     E->G.assign(count, 1);
+    E->own.assign(count, 0);
     E->ctas = E->sm_count * 4;
     std::memset(E->members.data(), 0, sizeof(vl::EnsMember) * count);
     int rc = E->precision == VL_FP64 ? upload_tables<double>(E->ctx) : upload_tables<float>(E->ctx);
@@ -737,6 +741,7 @@ VL_API int vl_ens_schedule(vl_ens *E, int32_t threads, int32_t ctas_per_sm, int3
         total += (double)c->cfg.nx * tiles_of(c) * n * n * n;
     }
     const double target = total / ((double)E->ctas * items_per_cta);
+    E->own.assign(count, 0);
     for (int i = 0; i < count; ++i) {
         const vl_ctx *c = E->ctx[i];
         const double n = c->cfg.n;
@@ -755,7 +760,7 @@ VL_API int vl_ens_schedule_by_order(vl_ens *E, int32_t items_per_cta, uint32_t n
     // members launched through their own contexts: those of the orders in the mask, or with
     // VL_ENS_NATIVE_AUTO those whose context stages its tiles by TMA (fragment kernel, TMA
     // kernel, the generic kernel's TMA form), which beat the ensemble's register-pencil body
-    std::vector<char> native(count, 0);
+    std::vector<char> native(count, 0), own(count, 0);
     for (int i = 0; i < count; ++i) {
         const vl_ctx *c = E->ctx[i];
         if (native_orders == VL_ENS_NATIVE_AUTO)
@@ -765,14 +770,16 @@ VL_API int vl_ens_schedule_by_order(vl_ens *E, int32_t items_per_cta, uint32_t n
             native[i] = (native_orders >> c->cfg.n) & 1u;
     }
     double total[vl::NMAX + 1] = {};
-    double native_dof = 0.0;   // interior values of the native members
+    double native_dof = 0.0, most = 0.0;   // interior values of the native members, of the largest
     bool any_native[vl::NMAX + 1] = {};
     for (int i = 0; i < count; ++i) {
         const vl_ctx *c = E->ctx[i];
         const double n = c->cfg.n;
         if (native[i]) {
             any_native[c->cfg.n] = true;
-            native_dof += (double)c->cfg.nx * c->cfg.nu * c->cfg.nv * n * n * n;
+            const double dof = (double)c->cfg.nx * c->cfg.nu * c->cfg.nv * n * n * n;
+            native_dof += dof;
+            most = std::max(most, dof);
         }
         if (!native[i]) total[c->cfg.n] += (double)c->cfg.nx * tiles_of(c) * n * n * n;
     }
@@ -799,14 +806,21 @@ VL_API int vl_ens_schedule_by_order(vl_ens *E, int32_t items_per_cta, uint32_t n
     // its share of the work, 2 items_per_cta per resident CTA in all: long-lived CTAs of many tiles,
     // enough of them to even out the members' ends.  24 FP32 members of about 1.9M values: 0.65 ms per
     // step at 2 items per CTA on 32 streams, 1.10 ms with every launch sized for the whole device (2 to 3
-    // tiles per CTA) on 8 streams; 64 members 1.67 against 1.82 ms.
+    // tiles per CTA) on 8 streams; 64 members 1.67 against 1.82 ms.  A member that would get more than a wave
+    // is sized for the whole device (FP64 16x20x20 n = 6 alone 92 us per step with its share, 62 so); where one
+    // has most of the work, all are: the others' few long CTAs would wait for its wave and run on after it
+    // (32x50x50 n = 8 beside two of 1% 752 against 640).
     // Other members: about items_per_cta items of similar cost per CTA of their order's kernel.
+    const bool dominated = 2.0 * most > native_dof;
     for (int i = 0; i < count; ++i) {
         const vl_ctx *c = E->ctx[i];
         if (native[i]) {
             const double share = (double)c->cfg.nx * c->cfg.nu * c->cfg.nv * c->cfg.n * c->cfg.n * c->cfg.n / native_dof;
             const int G = (int)(share * 2 * items_per_cta * c->stage_slots / c->cfg.nx + 0.5);
             E->G[i] = std::max(1, std::min(G, c->stage_tiles));
+            // (a member whose share asks for more takes the grids that its context has for the device alone)
+            own[i] = dominated || E->G[i] >= c->stage_grid_g;
+            if (own[i]) E->G[i] = c->stage_grid_g;
             continue;
         }
         const double n = c->cfg.n;
@@ -830,6 +844,7 @@ VL_API int vl_ens_schedule_by_order(vl_ens *E, int32_t items_per_cta, uint32_t n
     }
     E->groups = groups;
     E->native = native;
+    E->own = own;
     E->by_order = true;
     E->dirty = true;
     return VL_OK;
