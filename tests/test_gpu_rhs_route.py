@@ -1,7 +1,7 @@
 """FP32 order 3 on rows that no tensor copy takes: a right-hand side alone runs on the register-pencil kernel
-where the line form's tiles would be mostly empty (rows of 29 elements in tiles of 28), on the line form
-elsewhere; the stages always on the line form.  Told apart by their rounding: the same bits as the forced
-kernel, and other bits than the other one."""
+where the line form's tiles would be too empty (rows of 29 elements in tiles of 28) and not all resident at
+once, on the line form elsewhere; the stages always on the line form.  Told apart by their rounding: the
+same bits as the forced kernel, and other bits than the other one."""
 import pytest
 import torch
 
@@ -11,8 +11,11 @@ from test_gpu_line_kernel import TOL, _context, _inputs
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("res,pencil", [((2, 5, 29), True), ((3, 4, 31), True), ((2, 6, 57), True), ((1, 5, 1), True),
-                                        ((2, 5, 25), False), ((2, 4, 27), False), ((2, 3, 83), False)])
+@pytest.mark.parametrize("res,pencil", [((64, 40, 29), True), ((48, 50, 31), True), ((64, 40, 57), True),
+                                        ((64, 80, 1), True), ((64, 40, 67), True), ((64, 30, 89), True),
+                                        ((64, 40, 25), False), ((48, 50, 27), False), ((64, 40, 83), False),
+                                        ((64, 40, 45), False), ((64, 20, 117), False),
+                                        ((2, 5, 29), False), ((1, 5, 1), False)])
 def test_order_3(cuda, res, pencil, monkeypatch):
     from vlasov1d2v_b200 import _lib, problem
 

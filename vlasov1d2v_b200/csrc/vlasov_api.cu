@@ -1257,14 +1257,17 @@ int vl_ctx_create(const vl_config *cfg, vl_ctx **out) {
         c->stage_grid_g1 = line_grid(lo1);
         slots1 = c->sm_count * lo1;
         // FP32 n = 3: the line form's tiles of 28 v elements leave much of a row's last tile empty where nv is
-        // just above a multiple.  A right-hand side then runs on the register-pencil kernel (tiles of 10):
-        // 64x57x29 16.0 us against 24.4, 32x61x57 16.3 against 17.9; 32x61x85 24.4 either way, 16x31x25 4.5
-        // against 3.7.  The loop's stages stay, for the field solve inside them (64x72x57 168 us per step
+        // just above a multiple.  A right-hand side then runs on the register-pencil kernel (tiles of 10), of
+        // whose tiles 2.4 take as long as one of the line form: 64x57x29 (3 of them against 2) 16.0 us against
+        // 24.4, 64x101x39 (4, 2) 33.3 against 41.1, 64x101x89 (9, 4) 80.4 against 84.0, 64x101x67 (7, 3) 60.7
+        // against 63.2; not 64x101x45 (5, 2) 41.6 against 41.0, 64x101x117 (12, 5) 106 against 98, 64x101x25
+        // (3, 1) 27.0 against 22.4.  A grid whose line-form tiles are all resident at once stays too (8x12x29
+        // 3.3 against 4.0), and the loop's stages do, for the field solve inside them (64x72x57 168 us per step
         // against 184 on the register-pencil kernel).
-        if (!forced && !d && n == 3 && general == VL_STAGE_PENCIL && 4 * cfg->nv < 3 * ept * ((cfg->nv + ept - 1) / ept)) {
-            const int pt = 32 / n, ptiles = cfg->nu * ((cfg->nv + pt - 1) / pt);
+        const int pt = 32 / n, ptiles = cfg->nu * ((cfg->nv + pt - 1) / pt);
+        if (!forced && !d && n == 3 && general == VL_STAGE_PENCIL && 5 * ptiles < 12 * lt &&
+            lt * cfg->nx > slots1)
             c->rhs_pencil_g = wave_grid(ptiles, cfg->nx, c->sm_count * stage_occupancy<float>(n, false, false, false, false));
-        }
     }
     {
         // the field solve inside the stage kernels: tables, a kernel that has the prologue, room for the
